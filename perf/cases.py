@@ -303,7 +303,8 @@ def tolerance(case):
     if prec == "fp64":
         return {"rel": 1e-13, "max": 1e-11}
     if prec == "fp32":
-        return {"rel": 1e-6 if kind == "ek2d" else 5e-6, "max": 1e-3, "differ": 1e-4}
+        return {"rel": 1e-6, "max": 1e-3} if kind == "ek2d" else {"rel": 5e-6, "max": 0.05,
+                                                                 "differ": 1e-4}
     if kind == "ek2d":
         return {"rel": 4e-4, "max": 0.05} if prec == "fp16" else {"rel": 4e-3, "max": 0.2}
     return {"rel": 1.5e-2, "max": 0.5, "differ": 2e-3}
