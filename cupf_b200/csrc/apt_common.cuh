@@ -73,6 +73,13 @@ struct StepArgs {
   // (may be NULL): [0] entries aliased into the next point's slot 0 (s < 6),
   // [1] entries dropped at the last point (s == 6)
   unsigned long long* overflows;
+  // Slot maps (apt_step.cuh; NULL = none kept, every cell merged every step): NUM_PF
+  // planes of one word per cell, slot_stride words each, in the pair planes' layout.
+  // redo_in / redo_out: per cell, non-zero where a list its stencil reads changed in
+  // `in` / is changed by this step in `out`.
+  uint32_t* map;
+  uint8_t* redo_in;
+  uint8_t* redo_out;
   long long wait_limit;  // SM cycles a stage wait may spin before the step gives up
 };
 
@@ -112,6 +119,29 @@ __host__ __device__ __forceinline__ int bc_map(int c, int fn, int bc) {
   if (c == 0) return bc == 0 ? 2 : fn - 2;
   if (c == fn - 1) return bc == 0 ? fn - 3 : 1;
   return c;
+}
+
+// Mark the cells whose stencil reads cell (i, j, k): itself, its interior face
+// neighbours, and the cells beside a halo cell that the boundary map sources from
+// it.  redo: one byte per cell in the pair planes' layout.
+__host__ __device__ __forceinline__ void mark_readers(uint8_t* redo, int i, int j, int k, int fnx,
+                                                      int fny, int fnz, int xp, int bcX, int bcY,
+                                                      int bcZ) {
+  const long long plane = (long long)xp * fny;
+  uint8_t* c = redo + (long long)k * plane + (long long)j * xp + i;
+  c[0] = 1;
+  if (i > 1) c[-1] = 1;
+  if (i < fnx - 2) c[1] = 1;
+  if (j > 1) c[-xp] = 1;
+  if (j < fny - 2) c[xp] = 1;
+  if (k > 1) c[-plane] = 1;
+  if (k < fnz - 2) c[plane] = 1;
+  if (bc_map(0, fnx, bcX) == i) c[1 - i] = 1;
+  if (bc_map(fnx - 1, fnx, bcX) == i) c[fnx - 2 - i] = 1;
+  if (bc_map(0, fny, bcY) == j) c[(long long)(1 - j) * xp] = 1;
+  if (bc_map(fny - 1, fny, bcY) == j) c[(long long)(fny - 2 - j) * xp] = 1;
+  if (bc_map(0, fnz, bcZ) == k) c[(1 - k) * plane] = 1;
+  if (bc_map(fnz - 1, fnz, bcZ) == k) c[(fnz - 2 - k) * plane] = 1;
 }
 
 enum ErrCode { ERR_TMA_TIMEOUT = 1 };

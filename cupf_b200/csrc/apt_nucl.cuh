@@ -33,6 +33,10 @@ struct NuclArgs {
   int* count;           // nucleation events (accumulated)
   // quiet-item flags of the buffer written (NULL = none kept): the items a
   // nucleus reaches are marked not quiet; tile tw x th cells, z chunk zc
+  // change marks of the buffer written (NULL = none kept): a nucleus changes the
+  // id lists of its cells (mark_readers, apt_step.cuh)
+  uint8_t* redo;
+  int bcX, bcY, bcZ;
   uint8_t* quiet;
   int tw, th, zc, ntx, nty;
 };
@@ -136,6 +140,9 @@ __global__ void nucleate_kernel(typename S::T* buf, NuclArgs a) {
           const typename S::T old = buf[o];
           // `ph > -0.9999f` (a float literal, APTPhaseField.cu:524) == v > kDrop
           buf[o] = S::make(v, v > kDrop ? id : S::id(old));
+          if (a.redo && v > kDrop)
+            mark_readers(a.redo, gi + di, gj + dj, gk + dk, a.fnx, a.fny, a.fnz, a.xp, a.bcX, a.bcY,
+                         a.bcZ);
         }
     if (a.quiet) {
       for (int qz = (gk - a.pts - 1) / a.zc; qz <= (gk + a.pts - 1) / a.zc; ++qz)

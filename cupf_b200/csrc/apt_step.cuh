@@ -22,13 +22,21 @@
 // followed by a fill of the halo.  Halo edges and corners, which no 7-point
 // stencil reads, are not maintained by the step.
 //
-// After a plane lands, each cell of its tile gets a slot-occupancy bit mask
-// (bit p set when slot p holds an id).  The merge then visits only occupied
-// slots of the 7 stencil points, in the reference's order (D,B,L,C,R,T,U) x
-// slot, and records for every stencil point which source slot feeds which
-// output slot (4-bit codes), so the per-slot update reads exactly the values
-// the reference's local_phs array would hold, including its aliasing write on
-// merge overflow (local_phs[s][NUM_PF] == local_phs[s+1][0]).
+// Slot maps.  An output slot j of a cell holds one grain; the slot where each of
+// the 7 stencil points holds that grain follows from the points' ordered id
+// lists alone (the first-seen merge in the reference's order (D,B,L,C,R,T,U) x
+// slot).  It is kept per cell as one word per output slot, the slot map: 4 bits
+// per point, NUM_PF where the point lacks the grain.  The lists change seldom (a
+// front or tail crossing the cell), so the map belongs to the simulation's state
+// beside the pairs: a step merges again only the cells whose own or face
+// neighbours' lists changed in the step before.  Whoever changes a cell's list
+// marks the cells that read it (mark_readers) for the next step; whoever replaces
+// the whole state invalidates every map.  Merges are done by the warp together,
+// four cells a pass with a lane per stencil point, so a few scattered cells do not
+// hold up a warp's other lanes.
+//
+// The reference's aliasing write on merge overflow (local_phs[s][NUM_PF] ==
+// local_phs[s+1][0]) is restated: such cells are merged every step.
 #pragma once
 
 #include "apt_storage.cuh"
@@ -37,7 +45,9 @@
 namespace cupf {
 
 constexpr int TX = 32;
-constexpr int STAGES = 5;
+// Three planes in use and one in flight; a stage also holds a row of empty pairs
+// (slot NUM_PF, never written by the loads), which an absent grain's code reads.
+constexpr int STAGES = 4;
 
 // Column-tile heights the step is built for (the box height is TY + 2 cells; the
 // box width is the storage format's kBW).
@@ -52,42 +62,31 @@ struct StepSmem {
   static constexpr int BW = S::kBW;
   static constexpr int BH = TY + 2;
   static constexpr int BCELLS = BW * BH;
-  static constexpr int kBoxBytes = NP * BCELLS * S::kBytes;      // bytes one TMA plane load delivers
-  static constexpr int kStageBytes = (kBoxBytes + 127) & ~127;  // stage stride (TMA dst: 128 B aligned)
+  static constexpr int kBoxBytes = NP * BCELLS * S::kBytes;  // bytes one TMA plane load delivers
+  // stage stride (TMA dst: 128 B aligned), with the row of empty pairs
+  static constexpr int kStageBytes = ((NP + 1) * BCELLS * S::kBytes + 127) & ~127;
   static constexpr int kStagePairs = kStageBytes / S::kBytes;
-  static constexpr int kMaskOff = STAGES * kStageBytes;
   // 16-bit pairs in 32x8 tiles: the centre plane's phi values decoded once per
-  // plane into FP32 (slot-major like a stage, plus one row of -1 that the absent
-  // code NP points at), read by the five stencil points in that plane.  Three
-  // CTAs per SM still fit; for 32x4 tiles the extra row would cost one.
+  // plane into FP32 (slot-major like a stage, plus the row of -1), read by the
+  // five stencil points in that plane.  Three CTAs per SM still fit; for 32x4
+  // tiles the extra row would cost one.
   static constexpr bool kDecode = S::kBytes == 4 && TY == 8;
-  static constexpr int kDecOff = (kMaskOff + STAGES * BCELLS * 2 + 15) & ~15;
+  static constexpr int kDecOff = STAGES * kStageBytes;
   static constexpr int kDecBytes = kDecode ? (NP + 1) * BCELLS * 4 : 0;
-  static constexpr int kBarOff = (kDecOff + kDecBytes + 7) & ~7;
-  // + abort word, issued count, item index, one occupancy flag per stage
-  static constexpr int kBytes = kBarOff + STAGES * 8 + 16 + STAGES * 4;
+  // per warp: the merged cells' words, merge results and alias words
+  static constexpr int kWordOff = kDecOff + kDecBytes;
+  static constexpr int kBarOff = kWordOff + TY * (NP + 2) * 32 * 4;
+  // + abort word, issued count, item index
+  static constexpr int kBytes = kBarOff + STAGES * 8 + 16;
 };
 
-// Per-slot update loop shape of a storage format: rolled for the 16-bit pairs,
-// unrolled over NUM_PF for FP32 (each measured faster for its format).
-template <class S>
-struct RolledSlots {
-  static constexpr bool value = S::kBytes == 4;
-};
+// Slot-map words: 4-bit slot code of stencil point s in bits 4s..4s+3; the top 4
+// bits of slot 0's word hold the cell's slot count, or one of these marks.
+constexpr uint32_t kMapCodes = 0x0FFFFFFFu;
+constexpr uint32_t kMapEveryStep = 0xEu;  // merge overflow: merge this cell every step
+constexpr uint32_t kMapInvalid = 0xFu;    // nothing known (also what a byte-wise fill with 0xFF leaves)
 
-template <int NP>
-using CodeMap = typename std::conditional<(NP <= 8), uint32_t, unsigned long long>::type;
-
-// Replace 4-bit field j of a code map with v (one bfi for 32-bit maps).
-__device__ __forceinline__ uint32_t nib_insert(uint32_t c, uint32_t v, int j) {
-  uint32_t r;
-  asm("bfi.b32 %0, %1, %2, %3, 4;" : "=r"(r) : "r"(v), "r"(c), "r"(4 * j));
-  return r;
-}
-__device__ __forceinline__ unsigned long long nib_insert(unsigned long long c, uint32_t v, int j) {
-  const int sh = 4 * j;
-  return (c & ~(0xFull << sh)) | ((unsigned long long)v << sh);
-}
+__device__ __forceinline__ uint32_t map_code(uint32_t w, int s) { return (w >> (4 * s)) & 0xFu; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -169,22 +168,20 @@ struct CtaSmem {
   using P = typename S::T;
   using Smem = StepSmem<NP, S, TY>;
   P* stages;
-  uint16_t* masks;
   float* dec;     // decoded centre plane (Smem::kDecode)
+  uint32_t* wbuf; // merged cells (Smem::kWordOff)
   uint64_t* bars;
   int* s_abort;   // global plane sequence number of the first failed wait, + 1
   int* s_issued;  // plane sequence numbers issued so far (written by thread 0)
-  int* s_item;    // work item handed to the CTA (batched kernel)
-  int* s_occ;     // per stage: some cell of the landed plane holds an id
+  int* s_item;    // work item handed to the CTA
   __device__ explicit CtaSmem(unsigned char* smem) {
     stages = reinterpret_cast<P*>(smem);
-    masks = reinterpret_cast<uint16_t*>(smem + Smem::kMaskOff);
     dec = reinterpret_cast<float*>(smem + Smem::kDecOff);
+    wbuf = reinterpret_cast<uint32_t*>(smem + Smem::kWordOff);
     bars = reinterpret_cast<uint64_t*>(smem + Smem::kBarOff);
     s_abort = reinterpret_cast<int*>(smem + Smem::kBarOff + STAGES * 8);
     s_issued = s_abort + 1;
     s_item = s_abort + 2;
-    s_occ = s_abort + 4;
   }
   __device__ void init() {
     if (threadIdx.x == 0) {
@@ -193,8 +190,11 @@ struct CtaSmem {
       *s_issued = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (Smem::kDecode)
-      for (int c = threadIdx.x; c < Smem::BCELLS; c += blockDim.x) dec[NP * Smem::BCELLS + c] = -1.0f;
+    for (int c = threadIdx.x; c < Smem::BCELLS; c += blockDim.x) {
+      for (int s = 0; s < STAGES; ++s)
+        stages[(size_t)s * Smem::kStagePairs + NP * Smem::BCELLS + c] = S::empty();
+      if (Smem::kDecode) dec[NP * Smem::BCELLS + c] = -1.0f;
+    }
     __syncthreads();
   }
   // After a timed-out wait no further loads are issued; before the CTA exits
@@ -217,21 +217,17 @@ struct CtaSmem {
 template <int NP, class S, int TY>
 __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArgs& a, int txi,
                                           int tyi, int zci, CtaSmem<NP, S, TY>& sm, int& qbase) {
-  using Map = CodeMap<NP>;
-  static_assert(NP <= 8, "slot codes are 4-bit fields of one 32-bit word");
+  static_assert(NP <= 8, "slot codes are 4-bit fields, merge entries 8 per stencil point");
   using Smem = StepSmem<NP, S, TY>;
   constexpr int NTHREADS = tile_threads<TY>();
   using P = typename S::T;
   constexpr int BW = Smem::BW;
   constexpr int BCELLS = Smem::BCELLS;
   constexpr bool kDec = Smem::kDecode;
-  // code of an absent source slot: NP (the decoded plane's row of -1) where the
-  // centre plane is decoded, else 0xF; 0xE marks the aliased overflow value
-  constexpr uint32_t kAbsent = kDec ? (uint32_t)NP : 0xFu;
+  constexpr unsigned FULL = 0xffffffffu;
   // offsets of the centre plane's stencil points B, L, C, R, T from the cell
   constexpr int ctr_off[7] = {0, -BW, -1, 0, 1, BW, 0};
   P* stages = sm.stages;
-  uint16_t* masks = sm.masks;
   uint64_t* bars = sm.bars;
   int* s_abort = sm.s_abort;
   int* s_issued = sm.s_issued;
@@ -239,6 +235,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
 
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
+  const int lane = tx;  // TX == warp size: a warp is one tile row
   const int x0 = 1 + TX * txi;  // first interior x of the tile
   const int y0 = 1 + TY * tyi;
   const int k_begin = 1 + a.zc * zci;
@@ -253,7 +250,6 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
     const int s = g % STAGES;
     const int zl = k_begin - 1 + q;
     const int zp = bc_map(zl, a.fnz, a.bcZ);
-    if (kDec) sm.s_occ[s] = 0;
     mbar_arrive_expect_tx(&bars[s], Smem::kBoxBytes);
     tma_load_plane(stages + (size_t)s * Smem::kStagePairs, tmap, &bars[s], x0 - 1, y0 - 1, zp);
     *s_issued = g + 1;
@@ -267,7 +263,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
     for (int q = 0; q < npre; ++q) issue(q);
   }
 
-  // Wait for plane q and compute the occupancy masks of its cells.
+  // Wait for plane q.
   auto land = [&](int q) {
     const int g = q0 + q;
     const int s = g % STAGES;
@@ -276,20 +272,8 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
       atomicCAS(s_abort, 0, g + 1);
       atomicExch(a.err, ERR_TMA_TIMEOUT);
     }
-    const P* st = stages + (size_t)s * Smem::kStagePairs;
-    uint32_t any = 0;
-    for (int c = tid; c < BCELLS; c += NTHREADS) {
-      uint32_t m = 0;
-#pragma unroll
-      for (int p = 0; p < NP; ++p) m |= (uint32_t)(S::id(st[p * BCELLS + c]) != -1) << p;
-      masks[s * BCELLS + c] = (uint16_t)m;
-      any |= m;
-    }
-    if (kDec && any) sm.s_occ[s] = 1;
   };
 
-  land(0);
-  land(1);
   // bit 0: this thread wrote a slot other than the exact empty pair (an occupied
   // slot, or one whose id was just dropped: it keeps its last phi) or left one
   // unwritten; bits 1 and 2: the same in the item's bottom and top plane
@@ -308,62 +292,201 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
   const int hdx1 = bc_map(a.fnx - 1, a.fnx, a.bcX) == gx ? a.fnx - 1 - gx : 0;
   const int hdy0 = bc_map(0, a.fny, a.bcY) == gy ? -gy * a.xp : 0;
   const int hdy1 = bc_map(a.fny - 1, a.fny, a.bcY) == gy ? (a.fny - 1 - gy) * a.xp : 0;
-  const bool halo_any = (hdx0 | hdx1 | hdy0 | hdy1) != 0;
+  // (false for a whole warp away from the faces)
+  const bool halo_any = __any_sync(FULL, valid && (hdx0 | hdx1 | hdy0 | hdy1) != 0);
   // the line profile and the liquid-start undercooling depend on z only: one
-  // evaluation per plane instead of one per cell
+  // evaluation per plane instead of one per cell (32 planes at a time, one a lane)
   const bool plane_T = a.use_iuc || a.thermalType == 0 || a.thermalType == 1;
   const float kLS = __uint_as_float(kLSFloatBits);
   const float kDrop = __uint_as_float(kDropFloatBits);
   const KineConst kc = kine_const(a.kin_delta);
+  // this lane's part of a warp's merges: stencil point lane % 8 (7: none) of the
+  // pass's cell lane / 8; offset in pairs from the point's plane to the first cell
+  // of the warp's row
+  const int m_grp = lane >> 3, m_pt = lane & 7;
+  const int m_off = (ty + 1) * BW + 1 +
+                    (m_pt == 1 ? -BW : m_pt == 2 ? -1 : m_pt == 4 ? 1 : m_pt == 5 ? BW : 0);
+  uint32_t* wbuf = sm.wbuf + ty * ((NP + 2) * 32);
 
+  // the next plane's word 0 and change marks, loaded a plane ahead
+  const long long cell0 = (long long)k_begin * plane_pairs + (long long)gy * a.xp + gx;
+  uint32_t next_w0 = kMapInvalid << 28;
+  uint8_t next_r0 = 0, next_r1 = 0;
+  auto prefetch = [&](long long cell) {
+    if (a.map) {
+      next_w0 = a.map[cell];
+      next_r0 = a.redo_in[cell];
+      next_r1 = a.redo_out[cell];
+    }
+  };
+  if (valid) prefetch(cell0);
+
+  float Up_lane = 0.0f;
+  land(0);
+  land(1);
   for (int k = k_begin; k < k_end; ++k) {
     const int qk = k - k_begin + 1;
-    float Up_plane = 0.0f;
-    if (plane_T) {
+    const long long cell = cell0 + (long long)(k - k_begin) * plane_pairs;
+    uint32_t w[NP];
+    w[0] = next_w0 & kMapCodes;
+    int n = (int)(next_w0 >> 28);
+    // a mark left in redo_out by an earlier step (the item was not computed since)
+    // counts too; a neighbour setting it for the next step meanwhile costs only a
+    // merge with the same result
+    const bool need = valid && (n > NP || next_r0 || next_r1);
+    const bool had_mark = next_r0 != 0;
+    if (!valid || need) n = 0;
+#pragma unroll
+    for (int j = 1; j < NP; ++j)
+      if (j < n) w[j] = a.map[j * ss + cell];
+    if (valid && k + 1 < k_end) prefetch(cell + plane_pairs);
+    if (plane_T && (qk & 31) == 1) {  // lane l: plane k + l
       float T;
-      tinterp(a, 0, 0, k, &T);
-      Up_plane = __fdiv_rn(T, a.L_cp);
+      tinterp(a, 0, 0, min(k + lane, a.fnz - 1), &T);
+      Up_lane = __fdiv_rn(T, a.L_cp);
     }
+    const float Up_plane = __shfl_sync(FULL, Up_lane, (qk - 1) & 31);
     land(qk + 1);
-    __syncthreads();
+    const int sD = (q0 + qk - 1) % STAGES, sC = (q0 + qk) % STAGES, sU = (q0 + qk + 1) % STAGES;
+    P* stC = stages + (size_t)sC * Smem::kStagePairs;
+    // every thread has finished the previous plane at this barrier
+    bool occ = true;
+    if (kDec)
+      occ = __syncthreads_or(n > 0 || need) != 0;
+    else
+      __syncthreads();
     if (tid == 0 && qk >= 2 && qk - 2 + STAGES < nplanes && !*s_abort) {
       fence_proxy_async();
       issue(qk - 2 + STAGES);
     }
-    const int sD = (q0 + qk - 1) % STAGES, sC = (q0 + qk) % STAGES, sU = (q0 + qk + 1) % STAGES;
-    // decode the centre plane's phi once (a plane without ids needs none: every
-    // code into it is then absent); every thread has finished the previous
-    // plane, the last reader of the decoded values, at the barrier above
+    // decode the centre plane's phi once (unless no cell reads it)
     if constexpr (kDec) {
-      if (sm.s_occ[sC]) {
+      if (occ) {
         // four pairs per thread and pass (a stage and the decoded plane start on
         // 16-byte boundaries; NP * BCELLS is a multiple of 4)
         static_assert((NP * BCELLS) % 4 == 0, "vector decode");
-        const uint4* st = reinterpret_cast<const uint4*>(stages + (size_t)sC * Smem::kStagePairs);
+        const uint4* st = reinterpret_cast<const uint4*>(stC);
         float4* d4 = reinterpret_cast<float4*>(sm.dec);
         for (int e = tid; e < NP * BCELLS / 4; e += NTHREADS) {
-          const uint4 w = st[e];
-          d4[e] = make_float4(S::phi(w.x), S::phi(w.y), S::phi(w.z), S::phi(w.w));
+          const uint4 v = st[e];
+          d4[e] = make_float4(S::phi(v.x), S::phi(v.y), S::phi(v.z), S::phi(v.w));
         }
         __syncthreads();
       }
     }
+    const P* plD = stages + (size_t)sD * Smem::kStagePairs;
+    const P* plU = stages + (size_t)sU * Smem::kStagePairs;
+
+    // ---- merge of the warp's marked cells: first-seen order over (D,B,L,C,R,T,U) x
+    // slot.  Eight lanes take a cell, lane s the list of point s; each turn places
+    // the first grain not placed yet, and every lane finds the slot it has in its
+    // own list.  The turns give a word per point; its transpose the words per slot.
+    uint32_t alias = 0xFFFFFFFFu;  // slot at point s-1 whose value sits in slot 0 of point s
+    bool force_mark = false;
+    uint32_t todo = __ballot_sync(FULL, need);
+    if (todo) {
+      const P* mp = (m_pt == 0 ? plD : m_pt == 6 ? plU : stC) + m_off;
+      do {
+        int src = -1;  // the pass's cells: the lowest four marked lanes
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          if (m_grp == g) src = __ffs(todo) - 1;
+          todo &= todo - 1;
+        }
+        const bool on = src >= 0 && m_pt < 7;
+        const P* mc = mp + max(src, 0);
+        int id[NP];
+        uint32_t un = 0;  // slots of this point's list whose grain is not placed yet
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          id[p] = S::id(mc[p * BCELLS]);
+          un |= (uint32_t)(id[p] != -1) << p;
+        }
+        if (!on) un = 0;
+        uint32_t codes = m_pt < 7 ? (uint32_t)NP * 0x11111111u : 0u;
+        uint32_t dup = 0;
+        int cnt = 0;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          const uint32_t act = __ballot_sync(FULL, un != 0);
+          if (!act) break;
+          const uint32_t mine = (act >> (8 * m_grp)) & 0xFFu;
+          const int cand = S::id(mc[(un ? __ffs(un) - 1 : 0) * BCELLS]);
+          const int gid = __shfl_sync(FULL, cand, 8 * m_grp + (mine ? __ffs(mine) - 1 : 0));
+          uint32_t m = 0;
+#pragma unroll
+          for (int p = 0; p < NP; ++p) m |= (uint32_t)(id[p] == gid) << p;
+          if (!mine || !on) m = 0;
+          un &= ~m;
+          // the last slot holding the id, as the reference's later write wins
+          if (m) codes -= ((uint32_t)NP - (31u - (uint32_t)__clz(m))) << (4 * j);
+          dup |= m & (m - 1);
+          cnt += mine != 0;
+        }
+        // an id repeated in the centre's list does not survive the step
+        uint32_t info = (uint32_t)cnt << 28;
+        if (__any_sync(FULL, un | (m_pt == 3 ? dup : 0u))) {
+          // merge overflow: local_phs[s][NUM_PF] aliases local_phs[s+1][0], which
+          // point s+1's own grain of slot 0 overwrites; past the array at s == 6
+          const uint32_t below = __shfl_up_sync(FULL, un, 1);
+          const bool spill = m_pt >= 1 && m_pt <= 6 && below && (codes & 0xFu) == (uint32_t)NP;
+          uint32_t al = 0xFFFFFFFFu;
+          if (spill) al = ~(0xFu << (4 * m_pt)) | ((31u - (uint32_t)__clz(below)) << (4 * m_pt));
+          // entries aliased (low byte) and dropped (second byte); a list that loses
+          // an overflowing or repeated grain of the centre (bit 16); overflow (bit 17)
+          uint32_t q = m_pt < 6 ? (uint32_t)__popc(un) : (uint32_t)__popc(un) << 8;
+          uint32_t f = (m_pt == 3 && (un | dup) ? 1u << 16 : 0u) | (un ? 1u << 17 : 0u);
+#pragma unroll
+          for (int d = 1; d < 8; d <<= 1) {
+            al &= __shfl_xor_sync(FULL, al, d);
+            q += __shfl_xor_sync(FULL, q, d);
+            f |= __shfl_xor_sync(FULL, f, d);
+          }
+          info |= q | f;
+          if (src >= 0 && m_pt == 7) wbuf[(NP + 1) * 32 + src] = al;
+        }
+        // transpose the eight lanes' 4-bit fields: lane j gets slot j's word
+#pragma unroll
+        for (int d = 4; d; d >>= 1) {
+          const uint32_t keep = d == 4 ? 0x0000FFFFu : d == 2 ? 0x00FF00FFu : 0x0F0F0F0Fu;
+          const uint32_t o = __shfl_xor_sync(FULL, codes, d);
+          codes = (m_pt & d) ? (codes & ~keep) | ((o >> (4 * d)) & keep)
+                             : (codes & keep) | ((o & keep) << (4 * d));
+        }
+        if (src >= 0) {
+          if (m_pt < NP) wbuf[m_pt * 32 + src] = codes;
+          if (m_pt == 7) wbuf[NP * 32 + src] = info;
+        }
+      } while (todo);
+      __syncwarp();
+      if (need) {
+        const uint32_t info = wbuf[NP * 32 + lane];
+        n = (int)(info >> 28);
+#pragma unroll
+        for (int j = 0; j < NP; ++j)
+          if (j < n) w[j] = wbuf[j * 32 + lane];
+        uint32_t mark0 = (uint32_t)n;
+        if (info & 0x3FFFFu) {
+          force_mark = (info >> 16) & 1u;
+          n_ovf += (info & 0xFFu) + ((info & 0xFF00u) << 8);
+          if (info & (1u << 17)) {
+            alias = wbuf[(NP + 1) * 32 + lane];
+            mark0 = kMapEveryStep;
+          }
+        }
+        if (a.map) {
+          a.map[cell] = (n ? w[0] : 0u) | (mark0 << 28);
+#pragma unroll
+          for (int j = 1; j < NP; ++j)
+            if (j < n) a.map[j * ss + cell] = w[j];
+          if (had_mark) a.redo_in[cell] = 0;
+        }
+      }
+      __syncwarp();  // the buffer is rewritten at the next plane
+    }
     if (!valid) continue;
 
-    const P* pD = stages + (size_t)sD * Smem::kStagePairs + c;
-    const P* pC = stages + (size_t)sC * Smem::kStagePairs + c;
-    const P* pU = stages + (size_t)sU * Smem::kStagePairs + c;
-    const P* pts[7] = {pD, pC - BW, pC - 1, pC, pC + 1, pC + BW, pU};
-    uint32_t mk[7];
-    mk[0] = masks[sD * BCELLS + c];
-    mk[1] = masks[sC * BCELLS + c - BW];
-    mk[2] = masks[sC * BCELLS + c - 1];
-    mk[3] = masks[sC * BCELLS + c];
-    mk[4] = masks[sC * BCELLS + c + 1];
-    mk[5] = masks[sC * BCELLS + c + BW];
-    mk[6] = masks[sU * BCELLS + c];
-
-    P* outp = gout + (long long)k * plane_pairs + (long long)gy * a.xp + gx;
+    P* outp = gout + cell;
     // write pair v to output slot j of this cell and to the halo cells it sources
     auto put = [&](int j, P v) {
       P* o = outp + j * ss;
@@ -375,127 +498,26 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
         if (hdy1) o[hdy1] = v;
       }
     };
-    bool clive = false;
-    const uint32_t any = mk[0] | mk[1] | mk[2] | mk[3] | mk[4] | mk[5] | mk[6];
-    if (any == 0) {
+    if (n == 0) {
       const P empty = S::empty();
 #pragma unroll
       for (int p = 0; p < NP; ++p) put(p, empty);
       continue;
     }
 
-    // ---- merge: first-seen order over (D,B,L,C,R,T,U) x slot
-    int L[NP];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) L[q] = -1;
-    int n = 0;
-    Map code[7];
-    float alias[7];
-#pragma unroll
-    for (int s = 0; s < 7; ++s) {
-      code[s] = kDec ? (Map)(0x11111111u * kAbsent) : ~(Map)0;
-      alias[s] = -1.0f;
-    }
-    bool has_alias = false;  // some point's slot 0 holds an aliased overflow value
-    // General visit of stencil point s: each occupied slot's id is looked up in
-    // the list and appended when new (APTPhaseField.cu:211-233).
-    auto merge_point = [&](int s) {
-      uint32_t m = mk[s];
-      while (m) {
-        const int p = __ffs(m) - 1;
-        m &= m - 1;
-        const P pr = pts[s][p * BCELLS];
-        const int id = S::id(pr);
-        int j = n;
-#pragma unroll
-        for (int q = NP - 1; q >= 0; --q)
-          if (L[q] == id) j = q;
-        if (j == n) {
-          if (n < NP) {
-#pragma unroll
-            for (int q = 0; q < NP; ++q)
-              if (q == n) L[q] = id;
-            ++n;
-          } else {
-            // local_phs[s][NUM_PF] aliases local_phs[s+1][0]; past the array at s == 6
-            if (s < 6) {
-              code[s + 1] = nib_insert(code[s + 1], 0xEu, 0);
-              alias[s + 1] = S::phi(pr);
-              has_alias = true;
-            }
-            n_ovf += s < 6 ? 1u : 0x10000u;
-            continue;
-          }
-        }
-        code[s] = nib_insert(code[s], (uint32_t)p, j);
-      }
-    };
-    // A point whose every occupied slot q holds the id already at list position
-    // q maps q to q and adds nothing to the list: the general visit finds each of
-    // its ids at q (the list holds distinct ids).  The centre and the point above
-    // nearly always satisfy this, because every cell's slot order is the
-    // first-seen order of its own neighbourhood, which starts with the column.
-    auto identity_point = [&](int s) -> bool {
-      const uint32_t m = mk[s];
-      bool ok = true;
-      Map occ = 0;
-#pragma unroll
-      for (int q = 0; q < NP; ++q)
-        if ((m >> q) & 1u) {
-          ok = ok && (S::id(pts[s][q * BCELLS]) == L[q]);
-          occ |= (Map)0xF << (4 * q);
-        }
-      if (ok) code[s] = (code[s] & ~occ) | ((Map)0x76543210u & occ);
-      return ok;
-    };
-    // The point below comes first: the list is empty, so its slot p can only meet
-    // the ids of its own lower slots (n <= p, and the list cannot overflow).
-    {
-      const uint32_t m = mk[0];
-#pragma unroll
-      for (int p = 0; p < NP; ++p) {
-        if (!((m >> p) & 1u)) continue;
-        const int id = S::id(pts[0][p * BCELLS]);
-        int j = n;
-#pragma unroll
-        for (int q = p - 1; q >= 0; --q)
-          if (L[q] == id) j = q;
-        if (j == n) {
-#pragma unroll
-          for (int q = 0; q <= p; ++q)
-            if (q == n) L[q] = id;
-          ++n;
-        }
-        code[0] = nib_insert(code[0], (uint32_t)p, j);
-      }
-    }
-    merge_point(1);
-    merge_point(2);
-    if (!identity_point(3)) merge_point(3);
-    merge_point(4);
-    merge_point(5);
-    if (!identity_point(6)) merge_point(6);
-
-    // Value of output slot j at stencil point s: kAbsent = absent (-1), 0xE = the
-    // aliased overflow value, which only ever lands in slot 0 (kAlias false: the
-    // caller knows no point of the cell has one).  The five points of the centre
-    // plane read the decoded plane where there is one.
-    auto fetch = [&](int s, int j, auto alias_tag) -> float {
-      constexpr bool kAlias = decltype(alias_tag)::value;
-      const uint32_t cd = (uint32_t)(code[s] >> (4 * j)) & 0xF;
-      const bool al = kAlias && j == 0 && cd == 0xEu;
-      if (kDec && s >= 1 && s <= 5) {
-        // the index stays inside the decoded plane for the alias code too
-        const float v = sm.dec[(al ? kAbsent : cd) * BCELLS + c + ctr_off[s]];
-        return al ? alias[s] : v;
-      }
-      if (al) return alias[s];
-      if (cd == kAbsent) return -1.0f;
+    const P* pC = stC + c;
+    const P* pts[7] = {plD + c, pC - BW, pC - 1, pC, pC + 1, pC + BW, plU + c};
+    // Value of a slot-map word's grain at stencil point s.  The five points of the
+    // centre plane read the decoded plane where there is one.
+    auto phi_at = [&](uint32_t wj, int s) -> float {
+      const uint32_t cd = s == 6 ? wj >> 24 : map_code(wj, s);
+      if (kDec && s >= 1 && s <= 5) return sm.dec[cd * BCELLS + c + ctr_off[s]];
       return S::phi(pts[s][cd * BCELLS]);
     };
-    using WithAlias = std::integral_constant<bool, true>;
-    using NoAlias = std::integral_constant<bool, false>;
-
+    const bool aliased = alias != 0xFFFFFFFFu;
+    auto alias_at = [&](int s) -> float {  // slot 0's value at point s, where it is an alias
+      return S::phi(pts[s - 1][map_code(alias, s) * BCELLS]);
+    };
     // phi + 1 at the centre for every slot (the repulsion sum's terms); the loops
     // over slots stop at n, so a warp runs only as many iterations as its
     // fullest cell
@@ -505,8 +527,9 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
       if (q >= n) break;
-      phc1[q] = __fadd_rn(fetch(3, q, WithAlias{}), 1.0f);
+      phc1[q] = __fadd_rn(phi_at(w[q], 3), 1.0f);
     }
+    if (aliased && map_code(alias, 3) != 0xFu) phc1[0] = __fadd_rn(alias_at(3), 1.0f);
 
     // rounding bits of this cell and step: keyed on the cell's reference-layout
     // index and the step number, so a simulation rounds the same alone or batched
@@ -522,27 +545,56 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
       Up = __fdiv_rn(T, a.L_cp);
     }
 
-    // New value of output slot j < n holding grain `id`.
-    auto update_slot = [&](int j, int id, auto alias_tag) -> P {
-      // orientation of the grain (APTPhaseField.cu:259-273): loads issued before
-      // the stencil values are gathered so their latency overlaps; ids are >= 0
-      // here (cupf_apt_set_slots rejects other negative ids) and the clamp only
-      // keeps a corrupted id from reading outside the tables
+    bool clive = false;
+    bool changed = force_mark;  // the cell's id list differs from the one it came in with
+    // New value of output slot j < n, slot-map word wj.
+    auto update_slot = [&](int j, uint32_t wj) -> P {
+      // the grain's id: at the centre if that holds it, else at another point (the
+      // row of empty pairs gives -1)
+      const uint32_t cC = map_code(wj, 3);
+      int id = S::id(pC[cC * BCELLS]);
+      // orientation of the grain (APTPhaseField.cu:259-273), used only where the
+      // centre holds it: loads issued before the stencil values are gathered so
+      // their latency overlaps; ids are >= 0 there (cupf_apt_set_slots rejects
+      // other negative ids) and the clamp only keeps an absent or corrupted id
+      // from reading outside the tables
       int tid2 = id;
       if (id > a.num_theta)  // id % num_theta + 1
         tid2 = id - (int)div_invariant((uint32_t)id, a.nt_magic, a.nt_sh1, a.nt_sh2) * a.num_theta + 1;
       const bool tab_ok = (unsigned)tid2 <= (unsigned)a.num_theta;
       const int ti = tab_ok ? tid2 : 0;
-      const float4 t_o = __ldg(a.orient + ti);  // {sint[ti], cost[ti], sint[ti+NG], cost[ti+NG]}
+      float4 t_o = __ldg(a.orient + ti);  // {sint[ti], cost[ti], sint[ti+NG], cost[ti+NG]}
       float ph7[7];
 #pragma unroll
-      for (int s = 0; s < 7; ++s) ph7[s] = fetch(s, j, alias_tag);
+      for (int s = 0; s < 7; ++s) ph7[s] = phi_at(wj, s);
+      if (id == -1) {
+#pragma unroll
+        for (int s = 0; s < 7; ++s)
+          if (s != 3) id = max(id, S::id(pts[s][(s == 6 ? wj >> 24 : map_code(wj, s)) * BCELLS]));
+      }
+      if (j == 0 && aliased) {
+#pragma unroll
+        for (int s = 1; s < 7; ++s)
+          if (map_code(alias, s) != 0xFu) ph7[s] = alias_at(s);
+      }
       float sina = 0.0f, cosa = 1.0f, sinb = 0.0f, cosb = 1.0f;
-      if (ph7[3] > kLS && tab_ok) {  // (double)phC > LS
-        sina = t_o.x;
-        cosa = t_o.y;
-        sinb = t_o.z;
-        cosb = t_o.w;
+      if (ph7[3] > kLS) {  // (double)phC > LS
+        // an aliased centre value belongs to another grain than slot 0's
+        int to = ti;
+        bool ok = tab_ok;
+        if (j == 0 && aliased && cC == (uint32_t)NP) {
+          to = id;
+          if (id > a.num_theta)
+            to = id - (int)div_invariant((uint32_t)id, a.nt_magic, a.nt_sh1, a.nt_sh2) * a.num_theta + 1;
+          ok = (unsigned)to <= (unsigned)a.num_theta;
+          t_o = __ldg(a.orient + (ok ? to : 0));
+        }
+        if (ok) {
+          sina = t_o.x;
+          cosa = t_o.y;
+          sinb = t_o.z;
+          cosb = t_o.w;
+        }
       }
       // repulsion sum over the other slots (APTPhaseField.cu:328-335): the
       // reference accumulates r += 0.25 (phi+1)(phi+1) with the product fused,
@@ -554,67 +606,38 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
       static_assert(Contract::REP == 1, "the scaled sum restates the fused form only");
       float rsum = 0.0f;
 #pragma unroll
-      for (int q = 0; q < NP; ++q) {
-        if (q >= n) break;
+      for (int q = 0; q < NP; ++q)  // past n the terms are +0
         if (q != j) rsum = __fmaf_rn(phc1[q], phc1[q], rsum);
-      }
       const float repul = __fmul_rn(0.25f, rsum);
       const float nv = slot_update(a, kc, ph7, sina, cosa, sinb, cosb, repul, Up);
-      const int oid = (nv < kDrop) ? -1 : id;  // (double)nv < -0.9999
+      const bool drop = nv < kDrop;  // (double)nv < -0.9999
+      const int oid = drop ? -1 : id;
+      // The list stays as it was only if every kept grain sat in this same slot and
+      // every dropped one was absent (a grain of any slot past n is one of the n).
+      changed |= cC != (drop ? (uint32_t)NP : (uint32_t)j);
       // slot j's rounding bits: the cell's hashed key times a distinct odd
       // constant per slot (a bijection of a uniform 32-bit value, one multiply)
       if (S::kStochastic) return S::make_sr(nv, oid, cell_key * ((uint32_t)(2 * j + 1) * 0x9E3779B9u));
       return S::make(nv, oid);
     };
-    if constexpr (RolledSlots<S>::value) {
-      static_assert(S::kBytes == 4, "the packed id queue holds 16-bit ids");
-      // 16-bit pairs: one loop body run to the cell's slot count (the smaller code
-      // and register footprint measured faster at three CTAs per SM)
+    // one loop body run to the cell's slot count (unrolled over NUM_PF it overruns the
+    // instruction cache: 165 against 142 us per step, FP32, 128x128x256, NUM_PF = 8)
 #pragma unroll
-      for (int j = 0; j < NP; ++j)
-        if (j >= n) put(j, S::empty());
-      if (upd) {
-        auto slots = [&](auto alias_tag) {
-          // the list's ids (16-bit in these formats) packed two to a word and
-          // shifted down one id per slot: slot j's id is always the low half
-          uint32_t w[(NP + 1) / 2];
-#pragma unroll
-          for (int q = 0; q < (NP + 1) / 2; ++q)
-            w[q] = __byte_perm((uint32_t)L[2 * q], 2 * q + 1 < NP ? (uint32_t)L[2 * q + 1] : 0u, 0x5410);
+    for (int j = 0; j < NP; ++j)
+      if (j >= n) put(j, S::empty());
+    if (upd) {
 #pragma unroll 1
-          for (int j = 0; j < n; ++j) {
-            const int id = (int)(short)(w[0] & 0xFFFFu);
+      for (int j = 0; j < n; ++j) {
+        const P v = update_slot(j, w[0]);
 #pragma unroll
-            for (int q = 0; q < (NP + 1) / 2 - 1; ++q) w[q] = __funnelshift_r(w[q], w[q + 1], 16);
-            w[(NP + 1) / 2 - 1] >>= 16;
-            const P v = update_slot(j, id, alias_tag);
-            clive |= !S::is_empty(v);
-            put(j, v);
-          }
-        };
-        // merge overflows are rare: a warp none of whose cells has an aliased
-        // value runs the loop without the alias checks
-        if (__any_sync(__activemask(), has_alias))
-          slots(WithAlias{});
-        else
-          slots(NoAlias{});
-      } else {
-        clive = true;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        if (j >= n) {
-          put(j, S::empty());
-        } else if (upd) {
-          const P v = update_slot(j, L[j], WithAlias{});
-          clive |= !S::is_empty(v);
-          put(j, v);
-        } else {
-          clive = true;  // the reference leaves the slot unwritten
-        }
+        for (int q = 0; q + 1 < NP; ++q) w[q] = w[q + 1];
+        clive |= !S::is_empty(v);
+        put(j, v);
       }
     }
+    if (!upd) clive = changed = true;  // the reference leaves the slots unwritten
+    if (changed && a.map)
+      mark_readers(a.redo_out, gx, gy, k, a.fnx, a.fny, a.fnz, a.xp, a.bcX, a.bcY, a.bcZ);
     if (clive) live |= 1u | (k == k_begin ? 2u : 0u) | (k == k_end - 1 ? 4u : 0u);
   }
 
@@ -651,12 +674,13 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
 // whole item's bit 0).  Every cell of such an item would be written as the empty
 // pair again.
 template <int TY>
-__device__ __forceinline__ bool item_quiet(const StepArgs& a, int txi, int tyi, int zci) {
+__device__ __forceinline__ bool item_quiet(const StepArgs& a, const uint8_t* quiet_in,
+                                           const uint8_t* quiet_out, int txi, int tyi, int zci) {
   const int per = a.ntx * a.nty;
   const int it = zci * per + tyi * a.ntx + txi;
-  if (!(a.quiet_out[it] & 1) || !(a.quiet_in[it] & 1)) return false;
+  if (!(quiet_out[it] & 1) || !(quiet_in[it] & 1)) return false;
   auto q = [&](int tx, int ty, int zc, int bit) {
-    return (a.quiet_in[zc * per + ty * a.ntx + tx] & bit) != 0;
+    return (quiet_in[zc * per + ty * a.ntx + tx] & bit) != 0;
   };
   const int x0 = 1 + TX * txi, x1 = min(x0 + TX - 1, a.fnx - 2);
   const int y0 = 1 + TY * tyi, y1 = min(y0 + TY - 1, a.fny - 2);
@@ -672,30 +696,47 @@ __device__ __forceinline__ bool item_quiet(const StepArgs& a, int txi, int tyi, 
          q(txi, (yl - 1) / TY, zci, 1) && q(txi, (yr - 1) / TY, zci, 1);
 }
 
-// Hand the CTA its next work item from the launch's atomic counter (-1 when
-// none is left).  After its last fetch each CTA counts itself done; the last one
-// resets both words, so the next launch (or graph replay) starts from zero.
-__device__ __forceinline__ int next_work_item(int* work, int nitems, int* s_item,
-                                              const int* err) {
-  __syncthreads();  // every thread has read the previous index
-  if (threadIdx.x == 0) {
-    int it = atomicAdd(work, 1);
-    // a CTA that gave up on a load set the error word: take no further items
-    // (read with the ticket, once per item, not per plane)
-    if (*(volatile const int*)err != 0) it = nitems;
-    if (it >= nitems) {
-      it = -1;
-      __threadfence();
-      if (atomicAdd(work + 1, 1) == (int)gridDim.x - 1) {
-        atomicExch(work, 0);
-        atomicExch(work + 1, 0);
-      }
+// The work items of a persistent launch: CTA b starts with item b; further items
+// come from the launch's atomic counter, which a launch with no more items than
+// CTAs never touches.  Otherwise each CTA counts itself done once it has drawn past
+// the end; the last one resets both words, so the next launch (or graph replay)
+// starts from zero.
+struct WorkItems {
+  int* work;
+  int nitems;
+  int* s_item;
+  const int* err;
+  int ticket;  // the first item, then -1 (draw from the counter) or nitems
+  __device__ WorkItems(int* work, int nitems, int* s_item, const int* err)
+      : work(work), nitems(nitems), s_item(s_item), err(err), ticket(blockIdx.x) {}
+  // The CTA's next item, -1 when none is left (every thread gets the same).
+  __device__ __forceinline__ int next() {
+    if (nitems <= (int)gridDim.x) {  // one item a CTA
+      const int it = ticket < nitems ? ticket : -1;
+      ticket = nitems;
+      return it;
     }
-    *s_item = it;
+    __syncthreads();  // every thread has read the previous index
+    if (threadIdx.x == 0) {
+      int it = ticket >= 0 ? ticket : (int)gridDim.x + atomicAdd(work, 1);
+      ticket = -1;
+      // a CTA that gave up on a load set the error word: take no further items
+      // (read with the ticket, once per item, not per plane)
+      if (*(volatile const int*)err != 0) it = nitems;
+      if (it >= nitems) {
+        it = -1;
+        __threadfence();
+        if (atomicAdd(work + 1, 1) == (int)gridDim.x - 1) {
+          atomicExch(work, 0);
+          atomicExch(work + 1, 0);
+        }
+      }
+      *s_item = it;
+    }
+    __syncthreads();
+    return *s_item;
   }
-  __syncthreads();
-  return *s_item;
-}
+};
 
 // One launch = one step of one simulation.  Persistent CTAs pull work items
 // (column tile x z chunk) from an atomic counter, z-chunk-major so the chunks
@@ -722,12 +763,13 @@ __global__ void __launch_bounds__(tile_threads<TY>(), step_min_blocks<NP, S, TY>
   const int per_chunk = a.ntx * a.nty;
   const int nitems = per_chunk * a.nzc;
   int qbase = 0;
+  WorkItems items(a.work, nitems, sm.s_item, a.err);
   for (;;) {
-    const int it = next_work_item(a.work, nitems, sm.s_item, a.err);
+    const int it = items.next();
     if (it < 0) break;
     const int zci = it / per_chunk;
     const int r = it - zci * per_chunk;
-    if (a.quiet_out && item_quiet<TY>(a, r % a.ntx, r / a.ntx, zci)) continue;
+    if (a.quiet_out && item_quiet<TY>(a, a.quiet_in, a.quiet_out, r % a.ntx, r / a.ntx, zci)) continue;
     step_item<NP, S, TY>(&tmap, a, r % a.ntx, r / a.ntx, zci, sm, qbase);
   }
   sm.drain();

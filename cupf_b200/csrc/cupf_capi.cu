@@ -97,6 +97,10 @@ struct cupf_apt_handle {
   // finest item grid (z chunks of one plane); all 0 = nothing known
   uint8_t* quiet[2] = {nullptr, nullptr};
   size_t quiet_cap = 0;
+  // slot maps of the step and their change marks per buffer (StepArgs::map,
+  // redo_in/out); NULL where the device had no room for them
+  uint32_t* map = nullptr;
+  uint8_t* redo[2] = {nullptr, nullptr};
   bool skip_quiet = true;
   long long wait_limit = kWaitCycles;  // stage-wait bound of the step kernel (SM cycles)
   bool zc_user = false;  // z chunk fixed by the caller (set_tuning or CUPF_ZC)
@@ -201,7 +205,7 @@ static void free_handle(cupf_apt_handle* h) {
                   h->xfer_ph, h->xfer_id, h->layer_sums, h->alpha_full, h->loss_area,
                   h->counts, h->first, h->qoi_part, h->nucl_status, h->nucl_count,
                   h->nucl_sphere, h->jcand, h->jcount, h->jdistinct, h->quiet[0], h->quiet[1],
-                  h->active_cells, h->overflows, h->z64};
+                  h->active_cells, h->overflows, h->z64, h->map, h->redo[0], h->redo[1]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->ev0) cudaEventDestroy(h->ev0);
@@ -332,6 +336,31 @@ static cupf_status invalidate_quiet(cupf_apt_handle* h) {
   for (int b = 0; b < 2; ++b)
     if (h->quiet[b]) CK(cudaMemsetAsync(h->quiet[b], 0, h->quiet_cap, h->stream));
   return CUPF_OK;
+}
+
+// Forget every cell's slot map (slot 0's words): after the state was replaced.
+static cupf_status invalidate_maps(cupf_apt_handle* h) {
+  if (h->map) CK(cudaMemsetAsync(h->map, 0xFF, (size_t)h->g.ss * sizeof(uint32_t), h->stream));
+  return CUPF_OK;
+}
+
+// Slot maps and change marks of the step (a quarter of the FP32 pair buffers'
+// size).  A grid whose pairs leave no room for them runs without: every cell is
+// then merged every step, with the same results.
+static cupf_status alloc_maps(cupf_apt_handle* h) {
+  const size_t cells = (size_t)h->g.ss;
+  if (cudaMalloc((void**)&h->map, cells * h->g.np * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc((void**)&h->redo[0], cells) != cudaSuccess ||
+      cudaMalloc((void**)&h->redo[1], cells) != cudaSuccess) {
+    cudaGetLastError();  // not an error of the call
+    for (void* p : {(void*)h->map, (void*)h->redo[0], (void*)h->redo[1]})
+      if (p) cudaFree(p);
+    h->map = nullptr;
+    h->redo[0] = h->redo[1] = nullptr;
+    return CUPF_OK;
+  }
+  for (int b = 0; b < 2; ++b) CK(cudaMemsetAsync(h->redo[b], 0, cells, h->stream));
+  return invalidate_maps(h);
 }
 
 // Resident CTAs per SM the step kernel is compiled for (step_min_blocks).
@@ -524,6 +553,7 @@ extern "C" cupf_status cupf_apt_create(const cupf_apt_params* p, const cupf_apt_
   TRY(cuda(cudaMemsetAsync(h->overflows, 0, 2 * sizeof(unsigned long long), h->stream), "memset"));
   TRY(cuda(cudaMalloc((void**)&h->layer_sums, p->fnz * sizeof(double)), "layer sums"));
   for (int b = 0; b < 2; ++b) TRY(make_tmap(h, b));
+  TRY(alloc_maps(h));  // last: takes only room the rest left
   const char* zc_env = getenv("CUPF_ZC");
   h->zc_user = zc_env != nullptr;
   set_zc(h, zc_env ? atoi(zc_env) : default_zc(h));
@@ -633,6 +663,7 @@ extern "C" cupf_status cupf_apt_init_from_argmax(cupf_apt_handle* h, const float
   for (int b = 0; b < 2; ++b)
     if (cupf_status st = fill_halo(h, b)) return st;
   if (cupf_status st = invalidate_quiet(h)) return st;
+  if (cupf_status st = invalidate_maps(h)) return st;
   CK(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream));  // a new state: no step has failed
   h->cur = 0;
   h->steps_done = 0;
@@ -684,6 +715,7 @@ extern "C" cupf_status cupf_apt_set_slots(cupf_apt_handle* h, const float* ph, c
   for (int b = 0; b < 2; ++b)
     if ((st = fill_halo(h, b))) return st;
   if ((st = invalidate_quiet(h))) return st;
+  if ((st = invalidate_maps(h))) return st;
   CK(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream));  // a new state: no step has failed
   h->cur = 0;
   h->steps_done = steps_done;
@@ -735,6 +767,9 @@ extern "C" cupf_status cupf_apt_step(cupf_apt_handle* h, int32_t nsteps,
       a.quiet_in = h->quiet[h->cur];
       a.quiet_out = h->quiet[h->cur ^ 1];
     }
+    a.map = h->map;
+    a.redo_in = h->redo[h->cur];
+    a.redo_out = h->redo[h->cur ^ 1];
     a.active_cells = h->active_cells;
     a.overflows = h->overflows;
     cupf_status st = launch_step(h, a, h->tmap[h->cur]);
@@ -950,6 +985,10 @@ static NuclArgs nucl_args(cupf_apt_handle* h, int use_iuc) {
   a.sphere = h->nucl_sphere;
   a.status = h->nucl_status;
   a.count = h->nucl_count;
+  a.redo = h->redo[h->cur];
+  a.bcX = p.bcX;
+  a.bcY = p.bcY;
+  a.bcZ = p.bcZ;
   a.quiet = h->quiet[h->cur];
   a.tw = TX;
   a.th = h->ty;
@@ -1127,6 +1166,7 @@ extern "C" cupf_status cupf_apt_move_domain(cupf_apt_handle* h, int32_t* tip_fro
       CK(cudaMemcpyAsync(h->quiet[h->cur], h->quiet[tmp], nq, cudaMemcpyDeviceToDevice, h->stream));
     if (swap && *moved > 1) CK(cudaMemsetAsync(h->quiet[h->cur ^ 1], 0, nq, h->stream));
     CK(cudaGetLastError());
+    if ((st = invalidate_maps(h))) return st;
   }
   // the current buffer's halo still holds the state before the move (and so does
   // the other's after a copy back)

@@ -87,6 +87,8 @@ struct Request {
   int* dalpha = nullptr;
   float* ddummy = nullptr;
   uint8_t* dquiet[2] = {nullptr, nullptr};  // quiet-item flags of each buffer
+  uint32_t* dmap = nullptr;                 // slot maps (StepArgs::map), or NULL
+  uint8_t* dredo[2] = {nullptr, nullptr};   // change marks of each buffer
   size_t bytes = 0;
   int zc = 64, ty = 8, ntx = 0, nty = 0, nzc = 0;
   // results
@@ -202,7 +204,7 @@ static cudaError_t pool_alloc(cupf_server* s, void** p, size_t n) {
 // server's stream that reads them).
 static void free_request_device(cupf_server* s, Request* r) {
   void* ptrs[] = {r->buf[0], r->buf[1], r->dx, r->dy, r->dz, r->dz64, r->dsint, r->dcost, r->dorient, r->dphi,
-                  r->dalpha, r->ddummy, r->dquiet[0], r->dquiet[1]};
+                  r->dalpha, r->ddummy, r->dquiet[0], r->dquiet[1], r->dmap, r->dredo[0], r->dredo[1]};
   for (void* p : ptrs)
     if (p) cudaFreeAsync(p, s->stream);
   r->buf[0] = r->buf[1] = nullptr;
@@ -211,6 +213,8 @@ static void free_request_device(cupf_server* s, Request* r) {
   r->dalpha = nullptr;
   r->ddummy = nullptr;
   r->dquiet[0] = r->dquiet[1] = nullptr;
+  r->dmap = nullptr;
+  r->dredo[0] = r->dredo[1] = nullptr;
 }
 
 static size_t request_bytes(const cupf_apt_params& p, int pair_bytes, int num_pf) {
@@ -220,6 +224,15 @@ static size_t request_bytes(const cupf_apt_params& p, int pair_bytes, int num_pf
   // quiet flags for the most items a tile shape gives (32x4 tiles, z chunks of 1)
   const size_t quiet = 2 * (size_t)((p.fnx - 2 + TX - 1) / TX) * ((p.fny - 2 + 4 - 1) / 4) * (p.fnz - 2);
   return 2 * xp * p.fny * p.fnz * num_pf * pair_bytes + L * 8 + quiet + 4096;
+}
+
+// Bytes of a request's slot maps and change marks.  They are not part of
+// request_bytes: a request is admitted without them where the budget has no room
+// (its cells are then merged every step, with the same results).
+static size_t map_bytes(const cupf_apt_params& p, int pair_bytes, int num_pf) {
+  const int palign = pair_bytes == 8 ? 2 : 4;
+  const size_t xp = (p.fnx + palign - 1) / palign * palign;
+  return xp * p.fny * p.fnz * ((size_t)num_pf * sizeof(uint32_t) + 2);
 }
 
 // Pick the work items' tile shape of a grid shape -- the column-tile height
@@ -328,6 +341,22 @@ static cupf_status admit(cupf_server* s, Request* r, int slot) {
     CK(cudaMemsetAsync(r->dquiet[b], 0, nq, st));
   }
   r->bytes = request_bytes(p, s->pair_bytes, np);
+  // slot maps where the budget holds them beside this and every queued request
+  {
+    const size_t extra = map_bytes(p, s->pair_bytes, np);
+    size_t want = s->used_bytes + r->bytes + extra;
+    for (int64_t q : s->queue) want += request_bytes(s->reqs[q]->p, s->pair_bytes, np);
+    if (want <= s->budget) {
+      const size_t cells = (size_t)r->g.ss;
+      CK(pool_alloc(s, (void**)&r->dmap, cells * np * sizeof(uint32_t)));
+      CK(cudaMemsetAsync(r->dmap, 0xFF, cells * sizeof(uint32_t), st));  // nothing known
+      for (int b = 0; b < 2; ++b) {
+        CK(pool_alloc(s, (void**)&r->dredo[b], cells));
+        CK(cudaMemsetAsync(r->dredo[b], 0, cells, st));
+      }
+      r->bytes += extra;
+    }
+  }
   // initial state in both buffers
   e = with_fmt(s->cfg.precision, [&](auto tag) -> cupf_status {
     using S = decltype(tag);
@@ -425,6 +454,9 @@ static cupf_status admit(cupf_server* s, Request* r, int slot) {
   bs.buf[1] = r->buf[1];
   bs.quiet[0] = r->dquiet[0];
   bs.quiet[1] = r->dquiet[1];
+  a.map = r->dmap;
+  bs.redo[0] = r->dredo[0];
+  bs.redo[1] = r->dredo[1];
   bs.steps = 0;
   bs.target = r->nsteps;
   bs.cur = 0;
@@ -560,7 +592,7 @@ static cupf_status rebuild(cupf_server* s) {
 #define CASE(N)                                                                                 \
   case N: {                                                                                     \
     int grid[2] = {0, 0};                                                                       \
-    const int bytes8 = StepSmem<N, S, 8>::kBytes, bytes4 = StepSmem<N, S, 4>::kBytes;           \
+    constexpr int bytes8 = batch_smem_bytes<N, S, 8>(), bytes4 = batch_smem_bytes<N, S, 4>();   \
     CK(cudaFuncSetAttribute(apt_batch_step_kernel<N, S, 8>,                                     \
                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes8));              \
     CK(cudaFuncSetAttribute(apt_batch_step_kernel<N, S, 4>,                                     \
