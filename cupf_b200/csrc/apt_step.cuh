@@ -763,6 +763,10 @@ __global__ void __launch_bounds__(tile_threads<TY>(), step_min_blocks<NP, S, TY>
   const int per_chunk = a.ntx * a.nty;
   const int nitems = per_chunk * a.nzc;
   int qbase = 0;
+  // launched before the previous step has ended (launch_dependent): nothing above reads
+  // what that writes
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
   WorkItems items(a.work, nitems, sm.s_item, a.err);
   for (;;) {
     const int it = items.next();

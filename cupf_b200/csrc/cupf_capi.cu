@@ -233,8 +233,7 @@ static cupf_status launch_step_np(cupf_apt_handle* h, const StepArgs& a, const C
   }
   const int nitems = h->ntx * h->nty * h->nzc;
   const int nblk = std::min(nitems, h->grid_cap > 0 ? h->grid_cap : resident[h->device & 63]);
-  apt_step_kernel<NP, S, TY><<<nblk, NTHREADS, bytes, h->stream>>>(m, a);
-  CK(cudaGetLastError());
+  CK(launch_dependent(h->stream, nblk, NTHREADS, bytes, apt_step_kernel<NP, S, TY>, m, a));
   return CUPF_OK;
 }
 
