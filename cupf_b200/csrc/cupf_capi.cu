@@ -104,6 +104,7 @@ struct cupf_apt_handle {
   bool skip_quiet = true;
   long long wait_limit = kWaitCycles;  // stage-wait bound of the step kernel (SM cycles)
   bool zc_user = false;  // z chunk fixed by the caller (set_tuning or CUPF_ZC)
+  bool ty_user = false;  // tile height fixed by the caller (set_tile)
   unsigned long long* active_cells = nullptr;
   unsigned long long* overflows = nullptr;  // merge overflows: [0] aliased, [1] dropped
   // read-back scratch (reference layout, num_pf * length), allocated on first use
@@ -363,14 +364,14 @@ static cupf_status alloc_maps(cupf_apt_handle* h) {
 }
 
 // Resident CTAs per SM the step kernel is compiled for (step_min_blocks).
-static int resident_per_sm(const cupf_apt_handle* h) {
+static int resident_per_sm(const cupf_apt_handle* h, int ty) {
   int r = 2;
   with_storage(h->prec, [&](auto tag) -> cupf_status {
     using S = decltype(tag);
     switch (h->g.np) {
 #define CASE(N)                                                                      \
   case N:                                                                            \
-    r = h->ty == 4 ? step_min_blocks<N, S, 4>() : step_min_blocks<N, S, 8>();        \
+    r = ty == 4 ? step_min_blocks<N, S, 4>() : step_min_blocks<N, S, 8>();           \
     break;
       CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
 #undef CASE
@@ -393,28 +394,45 @@ static int default_zc(cupf_apt_handle* h) {
   const long long tiles =
       (long long)((h->p.fnx - 2 + TX - 1) / TX) * ((h->p.fny - 2 + h->ty - 1) / h->ty);
   const int nz = h->p.fnz - 2;
-  const long long want = (5LL * resident_per_sm(h) * nsm + 1) / 2;
+  const long long want = (5LL * resident_per_sm(h, h->ty) * nsm + 1) / 2;
   for (int zc = 16; zc > 1; zc /= 2)
     if (tiles * ((nz + zc - 1) / zc) >= want) return zc;
   return 1;
 }
 
-// z chunk for a state whose grain ids occupy nz_active interior planes (those
-// within 10 planes of a plane holding an id: the tails the first steps grow):
-// the largest of 16, 8, 4, 2 that gives at least 2 work items per resident CTA
-// over those planes, else 1.  Quiet items cost next to nothing, so the items
-// that count are the ones the step computes.  Measured on line cases (B200,
-// NUM_PF = 8, FP32 and FP16, 64^3 to 256x256x512): within 6 % of the best chunk
-// of 16..1 on every case, where sizing by all items was up to 18 % off.
-static int zc_for_active(cupf_apt_handle* h, int nz_active) {
+// Work-item shape for a state whose grain ids occupy nz_active interior planes (those
+// within 10 planes of a plane holding an id: the tails the first steps grow).  Quiet
+// items cost next to nothing, so the items that count are the ones the step computes.
+// The lines, measured on line cases on a B200 (us per step, tile height / z chunk):
+//   tile height 4 where it keeps as many warps resident as 8 does (16-bit pairs, and
+//     FP32 but for NUM_PF = 5 and 8), for its finer items: 256x256x512 FP16 768
+//     (4/16) against 841 (8/8), 96^3 FP16 45 (4/2) against 53 (8/1), 117x75x139 FP32
+//     NUM_PF = 6 53 (4/4) against 64 (8/2); where it does not, 8 is faster (192^3 FP32
+//     NUM_PF = 8: 229 against 245), unless the 32x8 tiles leave CTAs without an item
+//     even at one plane each (24x24x32: 8.4 against 16.2);
+//   z chunk: the largest of 16, 8, 4, 2 that gives 2 (tile height 8) or 1.75 (4) items
+//     per resident CTA over the active planes, else 1: within 3 % of the best chunk of
+//     1..32 on those cases and on 128x128x256 and 192^3 FP16.
+static cupf_status choose_shape(cupf_apt_handle* h, int nz_active) {
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  const long long tiles =
-      (long long)((h->p.fnx - 2 + TX - 1) / TX) * ((h->p.fny - 2 + h->ty - 1) / h->ty);
-  const long long want = 2LL * resident_per_sm(h) * nsm;
-  for (int zc = 16; zc > 1; zc /= 2)
-    if (tiles * ((nz_active + zc - 1) / zc) >= want) return zc;
-  return 1;
+  auto tiles = [&](int ty) {
+    return (long long)((h->p.fnx - 2 + TX - 1) / TX) * ((h->p.fny - 2 + ty - 1) / ty);
+  };
+  const int r8 = resident_per_sm(h, 8), r4 = resident_per_sm(h, 4);
+  if (!h->ty_user) {
+    const int ty = 4 * r4 >= 8 * r8 || tiles(8) * nz_active < (long long)r8 * nsm ? 4 : 8;
+    if (ty != h->ty) {
+      h->ty = ty;
+      for (int b = 0; b < 2; ++b)
+        if (cupf_status st = make_tmap(h, b)) return st;
+    }
+  }
+  const long long want = (h->ty == 4 ? 7LL * r4 : 8LL * r8) * nsm / 4;
+  int zc = 16;
+  while (zc > 1 && tiles(h->ty) * ((nz_active + zc - 1) / zc) < want) zc /= 2;
+  set_zc(h, zc);
+  return CUPF_OK;
 }
 
 // Interior planes within 10 planes of a plane that holds an id (plane_any[k]
@@ -587,6 +605,7 @@ extern "C" cupf_status cupf_apt_set_tile(cupf_apt_handle* h, int32_t tile_y) {
   CK(cudaSetDevice(h->device));
   CK(cudaStreamSynchronize(h->stream));  // no step in flight reads the old maps
   h->ty = tile_y;
+  h->ty_user = true;
   for (int b = 0; b < 2; ++b) {
     const cupf_status e = make_tmap(h, b);
     if (e) return e;
@@ -651,7 +670,7 @@ extern "C" cupf_status cupf_apt_init_from_argmax(cupf_apt_handle* h, const float
             plane_any[k] = 1;
             break;
           }
-    set_zc(h, zc_for_active(h, active_planes(plane_any, h->p.fnz)));
+    if (cupf_status cs = choose_shape(h, active_planes(plane_any, h->p.fnz))) return cs;
   }
   CK(cudaMemcpyAsync(h->phi_m, phi, L * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->alpha_m, alpha, L * sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -702,7 +721,7 @@ extern "C" cupf_status cupf_apt_set_slots(cupf_apt_handle* h, const float* ph, c
               plane_any[k] = 1;
               break;
             }
-    set_zc(h, zc_for_active(h, active_planes(plane_any, h->p.fnz)));
+    if (cupf_status cs = choose_shape(h, active_planes(plane_any, h->p.fnz))) return cs;
   }
   cupf_status st = ensure_xfer(h);
   if (st) return st;

@@ -169,7 +169,8 @@ class APTSolver:
         abi.check(self.L.cupf_apt_set_tuning(self.h, int(z_chunk)))
 
     def set_tile(self, tile_y):
-        """Column-tile height of the step's work items: 8 (default) or 4."""
+        """Column-tile height of the step's work items, 8 or 4 (default: picked when a
+        state is loaded)."""
         abi.check(self.L.cupf_apt_set_tile(self.h, int(tile_y)))
 
     def set_wait_limit(self, cycles):

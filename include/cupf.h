@@ -301,7 +301,7 @@ cupf_status cupf_apt_time_steps(cupf_apt_handle* h, int32_t nsteps, float* ms);
 void* cupf_apt_stream(cupf_apt_handle* h);
 
 /* Launch shape of the step kernel: z_chunk = interior planes per CTA work item
- * (the column tile is fixed at 32 x 8).  No reference counterpart (the
+ * (a column tile of 32 x 8 or 32 x 4 cells).  No reference counterpart (the
  * reference marches every column over the whole height, APTPhaseField.cu:190).
  * Without this call (or the CUPF_ZC environment variable) the library picks the
  * chunk whenever a state is loaded (init_from_argmax, set_slots) from the
@@ -309,9 +309,11 @@ void* cupf_apt_stream(cupf_apt_handle* h);
 cupf_status cupf_apt_set_tuning(cupf_apt_handle* h, int32_t z_chunk);
 
 /* Column-tile height of the step's work items (no counterpart in the reference,
- * whose kernel uses 32x4 thread blocks): 8 (the default) or 4 rows of 32 cells.
- * Results are identical for both; only the speed differs (the server picks per
- * grid shape by timing both with the z chunk).  Resets the quiet-item flags. */
+ * whose kernel uses 32x4 thread blocks): 8 or 4 rows of 32 cells.  Without this
+ * call the library picks the height with the chunk whenever a state is loaded;
+ * after it, the given height stays.  Results are identical for both; only the
+ * speed differs (the server picks per grid shape by timing both with the z
+ * chunk).  Resets the quiet-item flags. */
 cupf_status cupf_apt_set_tile(cupf_apt_handle* h, int32_t tile_y);
 
 /* Quiet work items (on by default).  The step keeps, per work item and buffer, a
