@@ -108,29 +108,37 @@ EkArgs make_args(const cupf_ek2d_handle* h, int prestep, uint32_t step) {
   a.up_b = (dxd / W0) / h->lT_tilde;
   a.seed = (uint32_t)p.seed_val;
   a.step = step;
+  a.fc = flux_consts(a);
   return a;
 }
 
-// Rows each warp marches over: 32, halved (down to 8) while the grid would give
-// fewer than about two waves of resident warps (32 per SM at 8 warps per CTA).
+// Warps of a step launch at `rows` rows each (strips x row chunks).
+long long march_warps(const cupf_ek2d_handle* h, int rows) {
+  return (long long)((h->fnx - 2 + MW - 1) / MW) * ((h->fny - 2 + rows - 1) / rows);
+}
+
+// Rows each warp marches over: 32, halved (down to 2) while the grid would give
+// fewer than 16 warps per SM (half of what is resident).
 int march_rows(const cupf_ek2d_handle* h) {
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  const long long strips = (h->fnx - 2 + MW - 1) / MW;
   int rows = 32;
-  while (rows > 8 && strips * ((h->fny - 2 + rows - 1) / rows) < 2LL * 32 * nsm) rows /= 2;
+  while (rows > 2 && march_warps(h, rows) < 16LL * nsm) rows /= 2;
   return rows;
 }
 
 cupf_status launch_step(cupf_ek2d_handle* h, int prestep, uint32_t step) {
   EkArgs a = make_args(h, prestep, step);
   a.rows = h->rows;
-  const int nstrips = (h->fnx - 2 + MW - 1) / MW;
-  const dim3 grid((nstrips + MWARPS - 1) / MWARPS, (h->fny - 2 + a.rows - 1) / a.rows);
+  const unsigned grid = (unsigned)((march_warps(h, h->rows) + MWARPS - 1) / MWARPS);
   return with_ek_storage(h->prec, [&](auto tag) -> cupf_status {
     using S = decltype(tag);
-    ek2d_march_kernel<S><<<grid, MWARPS * 32, 0, h->stream>>>(a);
-    CK(cudaGetLastError());
+    if constexpr (sizeof(typename S::T) == 8)
+      CK(launch_dependent(h->stream, grid, MWARPS * 32, 0, ek2d_march_kernel<S>, a));
+    else if (prestep)
+      CK(launch_dependent(h->stream, grid, MWARPS * 32, 0, ek2d_march32_kernel<S, false>, a));
+    else
+      CK(launch_dependent(h->stream, grid, MWARPS * 32, 0, ek2d_march32_kernel<S, true>, a));
     return CUPF_OK;
   });
 }

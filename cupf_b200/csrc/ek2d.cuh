@@ -53,6 +53,26 @@ namespace ek2d {
 template <class T>
 __device__ __forceinline__ T tanh_t(T x);
 
+// The hardware approximations (about 1 ulp) as single instructions: subnormal inputs
+// and results, which the step's operands never are where it uses the result, go to
+// zero instead of through the scaling that the non-flushing forms add.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+constexpr float kLog2e = 1.44269504f;
+
 // FP32 / FP64: psi itself, as the reference stores it; phi = tanh(psi/sqrt2).
 template <class TT>
 struct StPlain {
@@ -133,7 +153,7 @@ struct StH16 {
   __device__ static float code(float ps) {
     const float x = fminf(fabsf(ps), kPsiClamp);
     if (!BF) return copysignf(x, ps);
-    return copysignf(__fdividef(2.0f, 1.0f + __expf(1.41421356f * x)), ps);
+    return copysignf(2.0f * rcp_approx(1.0f + ex2_approx((1.41421356f * kLog2e) * x)), ps);
   }
   __device__ static V st_ps(T ps) { return st(code(ps)); }
   __device__ static V st_ps_sr(T ps, uint32_t r) { return st_sr(code(ps), r); }
@@ -150,6 +170,19 @@ using StBF16 = StH16<true>;
 
 // ---- launch arguments ------------------------------------------------------
 
+// Constants of the FP32-arithmetic step (flux_consts), with the factors that multiply
+// a whole flux or difference folded together.  Part of the arguments: the arithmetic
+// reads them as constant operands instead of holding them in registers.
+struct FluxConsts {
+  float cosa, sina, a_s, ase, a12;
+  float j0, j1;      // jat/2 = (j0 + j1 U) (1 - phi^2) dpsi
+  float g0, g1;      // solute conductance g0 + g1 (phi_a + phi_b)
+  float dthi, dts;   // dt hi, 2 sqrt2 dt
+  float opk, nomk;   // tau_U = opk + nomk phi
+  float hi2, sqrt2, inv_sqrt2, nex, nlam;
+  float eps, eps4, k, dt, U0;
+};
+
 struct EkArgs {
   const void* in;     // three planes (psi, U, dpsi), each fny rows of `pitch` values
   void* out;
@@ -161,7 +194,37 @@ struct EkArgs {
   float noise_amp;    // dt_sqrt*hi*eta; 0 disables the noise term
   double up_a, up_b;  // Up of memory row j = up_a + j*up_b
   uint32_t seed, step;
+  FluxConsts fc;
 };
+
+inline FluxConsts flux_consts(const EkArgs& a) {
+  FluxConsts c;
+  c.cosa = a.cosa;
+  c.sina = a.sina;
+  c.a_s = a.a_s;
+  c.ase = a.a_s * a.epsilon;
+  c.a12 = a.a_12;
+  c.j0 = 0.25f;
+  c.j1 = 0.25f * (1.0f - a.k);
+  const float hd = a.hi * a.Dl_tilde * 0.5f;
+  c.g0 = 2.0f * hd;
+  c.g1 = -hd;
+  c.dthi = a.dt * a.hi;
+  c.dts = 2.0f * a.sqrt2 * a.dt;
+  c.opk = 1.0f + a.k;
+  c.nomk = a.k - 1.0f;
+  c.hi2 = a.hi * a.hi;
+  c.sqrt2 = a.sqrt2;
+  c.inv_sqrt2 = 1.0f / a.sqrt2;
+  c.nex = -0.25f * a.sqrt2;
+  c.nlam = -a.lamd * a.sqrt2;
+  c.eps = a.eps;
+  c.eps4 = 4.0f * a.eps;
+  c.k = a.k;
+  c.dt = a.dt;
+  c.U0 = a.U0;
+  return c;
+}
 
 template <class T>
 struct Consts {
@@ -194,21 +257,19 @@ __device__ __forceinline__ Consts<T> consts(const EkArgs& a) {
 
 // Math of the step.  FP64 storage uses correctly rounded double operations
 // throughout.  The FP32-arithmetic storages (FP32, FP16, BF16) use the
-// hardware approximations (reciprocal, reciprocal square root, 2^x; a few ulp
+// hardware approximations (reciprocal, reciprocal square root, 2^x; about an ulp
 // each), far below the per-step differences the model's own rounding makes,
 // and tanh from its exponential form tanh(x) = 1 - 2/(1 + e^(2x)) (exact limits
 // +-1 at large |x|; absolute error of a few 1e-7 near 0).
 template <>
 __device__ __forceinline__ float tanh_t<float>(float x) {
-  return 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * x));
+  return fmaf(-2.0f, rcp_approx(1.0f + ex2_approx((2.0f * kLog2e) * x)), 1.0f);
 }
 template <>
 __device__ __forceinline__ double tanh_t<double>(double x) {
   return tanh(x);
 }
-__device__ __forceinline__ float div_t(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double div_t(double a, double b) { return a / b; }
-__device__ __forceinline__ float rsqrt_t(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double rsqrt_t(double x) { return 1.0 / sqrt(x); }
 
 // |phi| strictly inside the interface band, as the reference's
@@ -298,6 +359,29 @@ __device__ __forceinline__ T jat_of(const Consts<T>& c, T U, T ph, T D) {
   return (T)0.5 * ((T)1 + c.omk * U) * ((T)1 - ph * ph) * D;
 }
 
+// Stored values of one cell's new psi, U and dpsi.
+template <class S, class T = typename S::T, class V = typename S::V>
+__device__ __forceinline__ void encode_cell(const EkArgs& a, bool merge, uint32_t step_key, int gi,
+                                            int gj, T psn, T Un, T dps, V& vps, V& vU, V& vD) {
+  const T U0 = (T)a.U0;
+  if (S::kSR) {
+    // one 32-bit draw per cell and step: its two 16-bit halves round the
+    // phase field and U independently; dpsi is rewritten from scratch every
+    // step, not accumulated, so it rounds to nearest
+    const uint32_t r = mix32((uint32_t)(gi + a.fnx * gj) ^ step_key);
+    if (merge) {
+      S::st_ps_U_sr(psn, Un - U0, r, vps, vU);
+    } else {
+      vps = S::st_ps_sr(psn, r);
+      vU = S::stU(Un, U0);
+    }
+  } else {
+    vps = S::st_ps(psn);
+    vU = S::stU(Un, U0);
+  }
+  vD = S::st(dps);
+}
+
 // One cell's update and stores (PF.cu:553-598): U' from the divergence of the
 // solute fluxes, then psi' with the new U, dpsi = rhs/tau_psi, the optional
 // noise term, and the stores with their halo copies.
@@ -334,23 +418,7 @@ __device__ __forceinline__ void cell_update(const EkArgs& a, const Consts<T>& c,
   }
   const T psn = psC + c.dt * dps + noise;
   V vps, vU, vD;
-  if (S::kSR) {
-    // one 32-bit draw per cell and step: its two 16-bit halves round the
-    // phase field and U independently; dpsi is rewritten from scratch every
-    // step, not accumulated, so it rounds to nearest
-    const uint32_t r = mix32((uint32_t)(gi + a.fnx * gj) ^ step_key);
-    if (merge) {
-      S::st_ps_U_sr(psn, Un - c.U0, r, vps, vU);
-    } else {
-      vps = S::st_ps_sr(psn, r);
-      vU = S::stU(Un, c.U0);
-    }
-    vD = S::st(dps);
-  } else {
-    vps = S::st_ps(psn);
-    vU = S::stU(Un, c.U0);
-    vD = S::st(dps);
-  }
+  encode_cell<S>(a, merge, step_key, gi, gj, psn, Un, dps, vps, vU, vD);
   put_with_halo(o_ps, o_U, o_D, a.pitch, a.fnx, a.fny, gj, gi, vps, vU, vD);
 }
 
@@ -365,8 +433,19 @@ __device__ __forceinline__ void cell_update(const EkArgs& a, const Consts<T>& c,
 // below it was computed in the previous row.  The next row's loads are issued a
 // row ahead of their use.  No shared memory, no barriers.
 constexpr int MW = 30;
-constexpr int MWARPS = 8;
+constexpr int MWARPS = 4;
+// The warps of the launch take (strip, row chunk) pairs in order, strips
+// fastest, whatever the grid's width: no idle warps beside a narrow grid.
+struct MarchPos {
+  int group, chunk;
+  bool on;
+};
+__device__ __forceinline__ MarchPos march_pos(int ngroups, int nchunks) {
+  const int w = blockIdx.x * MWARPS + (int)(threadIdx.x >> 5);
+  return MarchPos{w % ngroups, w / ngroups, w < ngroups * nchunks};
+}
 
+// FP64 storage: one strip a warp, scalar arithmetic.
 template <class S>
 __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
   using T = typename S::T;
@@ -380,13 +459,14 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
   V* o_U = o_ps + a.plane;
   V* o_D = o_U + a.plane;
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int x0 = 1 + (blockIdx.x * MWARPS + warp) * MW;  // first output column of the strip
-  if (x0 > a.fnx - 2) return;                              // whole warp: uniform
+  const int lane = threadIdx.x & 31;
+  const MarchPos pos = march_pos((a.fnx - 2 + MW - 1) / MW, (a.fny - 2 + a.rows - 1) / a.rows);
+  if (!pos.on) return;             // whole warp: uniform
+  const int x0 = 1 + pos.group * MW;  // first output column of the strip
   const int gi = x0 - 1 + lane;
   const bool col_ok = gi < a.fnx;
   const bool out_col = lane >= 1 && lane <= MW && gi <= a.fnx - 2;
-  const int y0 = 1 + blockIdx.y * a.rows;
+  const int y0 = 1 + pos.chunk * a.rows;
   const uint32_t step_key = mix32(a.step ^ (a.seed * 0x9E3779B9u));
 
   // raw values of the next row to decode, loaded one row ahead of their use so
@@ -442,6 +522,9 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
                     j_b, j_c, J, Uf);
   };
 
+  // launched before the previous step has ended: nothing above reads what that writes
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
   issue(y0 - 1);
   fetch_c();
   shift();
@@ -473,6 +556,162 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
       cell_update<S>(a, c, merge, step_key, gi, r, ps_b, ph_b, U_b, j_b, xJ, xJ_L, yJ_hi, yJ_lo, xU,
                      xU_L, yU_hi, yU_lo, Rph_b, Lph, ph_c, ph_a, Rps_b, Lps, ps_c, ps_a, o_ps, o_U,
                      o_D);
+  }
+}
+
+
+// ---- the FP32-arithmetic storages' march
+//
+// The same march with the constants folded (FluxConsts) and the shared parts of the
+// two edges and the update formed once: 1 - phi^2 and jat/2 are carried with a row,
+// one reciprocal root per edge serves the normal and the anisotropy's 1/m^2 (the
+// squared gradient is the same before and after the rotation), and the row's Up is
+// formed in FP64 once per row by one lane instead of by every lane.
+
+// edge_flux from the sums of the two cells' phi and jat/2 and the difference of
+// their U.
+template <bool kY, bool kMerge>
+__device__ __forceinline__ void edge_flux32(const FluxConsts& c, float psx, float psz, float phx,
+                                            float phz, float sph, float dU, float sj, float& J,
+                                            float& Uf) {
+  const float m = fmaf(phx, phx, phz * phz);
+  const bool on = m > c.eps;
+  const float r = on ? rsqrt_approx(m) : 0.0f;
+  const float ux = fmaf(c.cosa, phx, c.sina * phz), uz = fmaf(c.cosa, phz, -c.sina * phx);
+  const float ux2 = ux * ux, uz2 = uz * uz;
+  const float r2 = r * r, inv = r2 * r2;
+  const float q = fmaf(ux2, ux2, uz2 * uz2);
+  const float A = fmaf(q * inv, c.ase, on ? c.a_s : 1.0f);
+  const float Ap = (ux * uz) * (ux2 - uz2) * (inv * c.a12);  // -aptheta
+  J = A * (kY ? fmaf(A, psz, -Ap * psx) : fmaf(A, psx, Ap * psz));
+  if (kMerge) Uf = fmaf(sj, (kY ? phz : phx) * r, fmaf(c.g1, sph, c.g0) * dU);
+}
+
+template <class S, bool kMerge>
+__global__ void __launch_bounds__(MWARPS * 32) ek2d_march32_kernel(const __grid_constant__ EkArgs a) {
+  using V = typename S::V;
+  const FluxConsts& c = a.fc;
+  const V* in = static_cast<const V*>(a.in);
+  V* out = static_cast<V*>(a.out);
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const MarchPos pos = march_pos((a.fnx - 2 + MW - 1) / MW, (a.fny - 2 + a.rows - 1) / a.rows);
+  if (!pos.on) return;  // whole warp: uniform
+  // lanes past the grid load its last column and store none
+  const int gi = pos.group * MW + lane, li = min(gi, a.fnx - 1);
+  const bool out_col = lane >= 1 && lane <= MW && gi <= a.fnx - 2;
+  const bool rim_col = gi == 1 || gi == a.fnx - 2;  // some halo cell copies it
+  const int y0 = 1 + pos.chunk * a.rows, y1 = min(y0 + a.rows, a.fny - 1);
+  const uint32_t step_key = mix32(a.step ^ (a.seed * 0x9E3779B9u));
+  const float Up_lane = (float)(a.up_a + (double)(y0 + lane) * a.up_b);  // rows <= 32
+
+  // raw values of the next row, loaded one row ahead of their use so that the load
+  // latency overlaps the current row's arithmetic (rows past the grid: the last row)
+  V raw_ps, raw_U, raw_D;
+  auto issue = [&](int r) {
+    const V* p = in + (long long)min(r, a.fny - 1) * a.pitch + li;
+    raw_ps = p[0];
+    raw_U = p[a.plane];
+    raw_D = p[2 * a.plane];
+  };
+  auto right = [&](float v) { return __shfl_down_sync(FULL, v, 1); };
+  auto left = [&](float v) { return __shfl_up_sync(FULL, v, 1); };
+  // row r+1 ("c") and its right neighbour; row r ("b"); row r-1 ("a"); w = 1 - phi^2,
+  // j = jat/2
+  float ps_c, ph_c, U_c, w_c, j_c, Rps_c, Rph_c, RU_c, Rj_c;
+  float ps_b, ph_b, U_b, w_b, j_b, Rps_b, Rph_b, RU_b, Rj_b;
+  float ps_a, ph_a;
+  auto fetch_c = [&]() {  // decode the issued row into "c"
+    S::ld_pp(raw_ps, c.inv_sqrt2, ps_c, ph_c);
+    U_c = S::ldU(raw_U, c.U0);
+    w_c = fmaf(-ph_c, ph_c, 1.0f);
+    j_c = fmaf(c.j1, U_c, c.j0) * w_c * S::ld(raw_D);
+    Rps_c = right(ps_c);
+    Rph_c = right(ph_c);
+    if (kMerge) {
+      RU_c = right(U_c);
+      Rj_c = right(j_c);
+    }
+  };
+  auto shift = [&]() {
+    ps_a = ps_b;
+    ph_a = ph_b;
+    ps_b = ps_c; ph_b = ph_c; U_b = U_c; w_b = w_c; j_b = j_c;
+    Rps_b = Rps_c; Rph_b = Rph_c; RU_b = RU_c; Rj_b = Rj_c;
+  };
+  // plaquette means at (x+1/2, r+1/2) from rows b and c
+  auto plaq = [&](float& qs, float& qp) {
+    qs = (((ps_b + Rps_b) + ps_c) + Rps_c) * 0.25f;
+    qp = (((ph_b + Rph_b) + ph_c) + Rph_c) * 0.25f;
+  };
+  // y-edge (x, r+1/2) between rows b and c
+  auto yedge = [&](float qs, float qp, float& J, float& Uf) {
+    edge_flux32<true, kMerge>(c, qs - left(qs), ps_c - ps_b, qp - left(qp), ph_c - ph_b, ph_b + ph_c,
+                              U_c - U_b, j_b + j_c, J, Uf);
+  };
+
+  // launched before the previous step has ended: nothing above reads what that writes
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+  issue(y0 - 1);
+  fetch_c();
+  shift();
+  issue(y0);
+  fetch_c();
+  issue(y0 + 1);
+  float qs_hi, qp_hi;
+  plaq(qs_hi, qp_hi);
+  float yJ_hi, yU_hi = 0.0f;
+  yedge(qs_hi, qp_hi, yJ_hi, yU_hi);
+
+  V* o = out + (long long)y0 * a.pitch + gi;
+#pragma unroll 2
+  for (int r = y0; r < y1; ++r, o += a.pitch) {
+    shift();
+    fetch_c();     // row r+1, issued one row earlier
+    issue(r + 2);  // in flight during this row's arithmetic
+    const float qs_lo = qs_hi, qp_lo = qp_hi;
+    plaq(qs_hi, qp_hi);
+    // x-edge (x+1/2, r)
+    float xJ, xU = 0.0f;
+    edge_flux32<false, kMerge>(c, Rps_b - ps_b, qs_hi - qs_lo, Rph_b - ph_b, qp_hi - qp_lo,
+                               ph_b + Rph_b, RU_b - U_b, j_b + Rj_b, xJ, xU);
+    const float yJ_lo = yJ_hi, yU_lo = yU_hi;
+    yedge(qs_hi, qp_hi, yJ_hi, yU_hi);
+    const float dJ = (xJ - left(xJ)) + (yJ_hi - yJ_lo);
+    const float psx = Rps_b - left(ps_b), phx = Rph_b - left(ph_b);  // twice the central
+    const float psz = ps_c - ps_a, phz = ph_c - ph_a;                // differences
+    const float Up = __shfl_sync(FULL, Up_lane, r - y0);
+    float Un = U_b;
+    if (kMerge) {
+      const float dF = (xU - left(xU)) + (yU_hi - yU_lo);
+      Un = fmaf(fmaf(c.dts, j_b, dF * c.dthi), rcp_approx(fmaf(c.nomk, ph_b, c.opk)), U_b);
+    }
+    // psi with the new U (PF.cu:563-590); the anisotropy is the same of twice the gradient
+    const float ux = fmaf(c.cosa, phx, c.sina * phz), uz = fmaf(c.cosa, phz, -c.sina * phx);
+    const float ux2 = ux * ux, uz2 = uz * uz, m = ux2 + uz2;
+    const float A = m > c.eps4
+                        ? fmaf(fmaf(ux2, ux2, uz2 * uz2) * rcp_approx(m * m), c.ase, c.a_s)
+                        : 1.0f;
+    const float A2 = A * A;
+    const float g4 = fmaf(psx, psx, psz * psz);
+    const float lap = fmaf(A2 * ph_b * c.nex, g4, dJ);
+    const float rhs = fmaf(w_b * (Un + Up), c.nlam, fmaf(lap, c.hi2, ph_b * c.sqrt2));
+    const float tp = fmaxf(fmaf(c.nomk, Up, 1.0f), c.k);
+    const float dps = rhs * rcp_approx(tp * A2);
+    float psn = fmaf(c.dt, dps, ps_b);
+    if (!out_col) continue;
+    if (a.noise_amp != 0.0f && in_band(ph_b)) {
+      const Philox4 rn = philox4x32_10((uint32_t)gi, (uint32_t)r, a.step, 0x4E4F4953u, a.seed, 0x5EEDu);
+      psn += a.noise_amp * ((float)uniform01(rn.v[0]) - 0.5f);
+    }
+    V vps, vU, vD;
+    encode_cell<S>(a, kMerge, step_key, gi, r, psn, Un, dps, vps, vU, vD);
+    o[0] = vps;
+    o[a.plane] = vU;
+    o[2 * a.plane] = vD;
+    if (rim_col || r == 2 || r == a.fny - 3)
+      put_with_halo(out, out + a.plane, out + 2 * a.plane, a.pitch, a.fnx, a.fny, r, gi, vps, vU, vD);
   }
 }
 
