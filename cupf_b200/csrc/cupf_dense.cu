@@ -34,7 +34,8 @@ struct cupf_dense_handle {
   unsigned short* lid[2] = {nullptr, nullptr};
   float* lval[2] = {nullptr, nullptr};
   bool list_ok[2] = {false, false};  // lists describe the buffer's current content
-  unsigned long long* overflow = nullptr;
+  unsigned long long* overflow = nullptr;  // two counters: this step's and the next's
+  int ovf = 0;                             // the last step's
   float *x = nullptr, *y = nullptr, *z = nullptr, *orient = nullptr;
   std::vector<float> z_host;
   float* phi_m = nullptr;
@@ -98,7 +99,6 @@ cupf_status launch_step(cupf_dense_handle* h, float t) {
     CK(cudaGetLastError());
     h->list_ok[ci] = true;
   }
-  CK(cudaMemsetAsync(h->overflow, 0, sizeof(unsigned long long), h->stream));
   DenseArgs a;
   std::memset(&a, 0, sizeof(a));
   a.fnx = p.fnx;
@@ -127,9 +127,10 @@ cupf_status launch_step(cupf_dense_handle* h, float t) {
   a.lid_o = h->lid[co];
   a.lval_o = h->lval[co];
   a.reset_from_lists = h->list_ok[co] ? 1 : 0;
-  a.overflow = h->overflow;
-  dense_update_kernel<<<grd, blk, 0, h->stream>>>(a);
-  CK(cudaGetLastError());
+  h->ovf ^= 1;
+  a.overflow = h->overflow + h->ovf;
+  a.overflow_next = h->overflow + (h->ovf ^ 1);
+  CK(launch_dependent(h->stream, grd, blk, 0, dense_update_kernel, a));
   h->list_ok[co] = true;
   h->cur ^= 1;
   h->halo_ok[h->cur] = false;
@@ -203,8 +204,8 @@ extern "C" cupf_status cupf_dense_create(const cupf_apt_params* p, const cupf_ap
     TRY(cuda(cudaMalloc((void**)&h->lval[b], (size_t)kDenseListMax * h->len * sizeof(float)),
              "lists"));
   }
-  TRY(cuda(cudaMalloc((void**)&h->overflow, sizeof(unsigned long long)), "overflow counter"));
-  TRY(cuda(cudaMemsetAsync(h->overflow, 0, sizeof(unsigned long long), h->stream), "memset"));
+  TRY(cuda(cudaMalloc((void**)&h->overflow, 2 * sizeof(unsigned long long)), "overflow counter"));
+  TRY(cuda(cudaMemsetAsync(h->overflow, 0, 2 * sizeof(unsigned long long), h->stream), "memset"));
   if (in->x) TRY(upload(&h->x, in->x, p->fnx, h->stream));
   if (in->y) TRY(upload(&h->y, in->y, p->fny, h->stream));
   TRY(upload(&h->z, in->z, p->fnz, h->stream));
@@ -477,7 +478,7 @@ extern "C" cupf_status cupf_dense_overflow_cells(cupf_dense_handle* h, int64_t* 
   if (!h || !overflow_cells) return cupf_fail(CUPF_ERR_INVALID, "null argument");
   CK(cudaSetDevice(h->device));
   unsigned long long v = 0;
-  CK(cudaMemcpyAsync(&v, h->overflow, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(&v, h->overflow + h->ovf, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   *overflow_cells = (int64_t)v;
   return CUPF_OK;
