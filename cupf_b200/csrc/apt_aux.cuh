@@ -65,19 +65,6 @@ __global__ void fill_halo_kernel(typename S::T* buf, Grid g, int bcX, int bcY, i
   }
 }
 
-// The halo cells of every slot, copied from src to dst unchanged.
-template <class S>
-__global__ void copy_halo_kernel(const typename S::T* __restrict__ src, typename S::T* dst,
-                                 Grid g) {
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < halo_cells(g);
-       idx += (long long)gridDim.x * blockDim.x) {
-    int i, j, k;
-    halo_cell(idx, g, i, j, k);
-    const long long d = g.at(i, j, k);
-    for (int p = 0; p < g.np; ++p) dst[p * g.ss + d] = src[p * g.ss + d];
-  }
-}
-
 // set_minus1 + APTini_PF on both buffers (PhaseField.cu:51-57, APTPhaseField.cu:78-89):
 // every slot (-1, -1), then slot 0 = (phi, alpha) where phi > LS.  phi/alpha in
 // reference layout (index i + j*fnx + k*fnx*fny).
@@ -166,45 +153,74 @@ __global__ void import_kernel(typename S::T* buf, const float* __restrict__ ph,
 
 // Per-layer sum of phi over every slot and cell (halo included), one block per
 // layer, double accumulation in a fixed order (deterministic; the reference
-// accumulates with float atomics, PhaseField.cu:366-378).
+// accumulates with float atomics, PhaseField.cu:366-378).  A warp takes rows, its
+// lanes the cells of a row, with the slots' loads in flight together.
+constexpr int kLayerThreads = 1024;
 template <class S>
-__global__ void layer_sum_kernel(const typename S::T* __restrict__ buf, double* sums, Grid g) {
+__global__ void __launch_bounds__(kLayerThreads)
+    layer_sum_kernel(const typename S::T* __restrict__ buf, double* sums, Grid g) {
   const int k = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double acc = 0.0;
-  const long long n = (long long)g.fnx * g.fny;
-  for (int p = 0; p < g.np; ++p)
-    for (long long c = threadIdx.x; c < n; c += blockDim.x) {
-      const int i = (int)(c % g.fnx), j = (int)(c / g.fnx);
-      acc += (double)S::phi(buf[p * g.ss + g.at(i, j, k)]);
+  for (int j = warp; j < g.fny; j += kLayerThreads / 32) {
+    const typename S::T* row = buf + g.at(0, j, k);
+    for (int i = lane; i < g.fnx; i += 32) {
+      int p = 0;
+      for (; p + 4 <= g.np; p += 4) {
+        typename S::T v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = row[(p + u) * g.ss + i];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc += (double)S::phi(v[u]);
+      }
+      for (; p < g.np; ++p) acc += (double)S::phi(row[p * g.ss + i]);
     }
-  __shared__ double red[256];
+  }
+  __shared__ double red[kLayerThreads];
   red[threadIdx.x] = acc;
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+  for (int s = kLayerThreads / 2; s > 0; s >>= 1) {
     if ((int)threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
     __syncthreads();
   }
   if (threadIdx.x == 0) sums[k] = red[0];
 }
 
-// One-layer shift of the interior (APTmove_frame + APTcopy_frame,
-// APTPhaseField.cu:357-410): dst[k] = src[k+1] for k < fnz-2, top interior layer
-// (-1, -1).  Halo cells are not touched.
+// One layer of a domain move in one pass over the slots: the argmax of every cell
+// (collect_kernel), and the interior shifted down one plane into dst
+// (APTmove_frame, APTPhaseField.cu:357-410: dst[k] = src[k+1] for k < fnz-2, the top
+// interior layer (-1, -1)); with `halo` dst also takes src's halo cells unchanged.
+// One thread a cell: a block takes 32 x 8 cells of one plane (move_layer_blocks).
+inline unsigned move_layer_blocks(const Grid& g) {
+  return (unsigned)((g.fnx + 31) / 32) * (unsigned)((g.fny + 7) / 8) * (unsigned)g.fnz;
+}
 template <class S>
-__global__ void shift_kernel(const typename S::T* __restrict__ src, typename S::T* dst, Grid g) {
-  const int ni = g.fnx - 2, nj = g.fny - 2, nk = g.fnz - 2;
-  const long long total = (long long)ni * nj * nk * g.np;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    long long r = idx;
-    const int i = 1 + (int)(r % ni);
-    r /= ni;
-    const int j = 1 + (int)(r % nj);
-    r /= nj;
-    const int k = 1 + (int)(r % nk);
-    const int p = (int)(r / nk);
-    const long long d = p * g.ss + g.at(i, j, k);
-    dst[d] = (k < g.fnz - 2) ? src[p * g.ss + g.at(i, j, k + 1)] : S::empty();
+__global__ void move_layer_kernel(const typename S::T* __restrict__ src, typename S::T* dst,
+                                  float* phi, int* alpha, Grid g, int halo) {
+  const int nbx = (g.fnx + 31) / 32, nby = (g.fny + 7) / 8, t = (int)(blockIdx.x % (nbx * nby));
+  const int i = t % nbx * 32 + (threadIdx.x & 31), j = t / nbx * 8 + (threadIdx.x >> 5);
+  const int k = (int)(blockIdx.x / (nbx * nby));
+  if (i >= g.fnx || j >= g.fny) return;
+  const bool inner = i > 0 && i < g.fnx - 1 && j > 0 && j < g.fny - 1 && k > 0 && k < g.fnz - 1;
+  const long long d = g.at(i, j, k);
+  const long long to = inner ? (k > 1 ? d - g.plane() : -1) : (halo ? d : -1);
+  const bool top = inner && k == g.fnz - 2;
+  typename S::T best{};
+  float bv = 0.0f;
+  for (int p = 0; p < g.np; ++p) {
+    const typename S::T v = src[p * g.ss + d];
+    const float f = S::phi(v);
+    if (p == 0 || f > bv) {
+      best = v;
+      bv = f;
+    }
+    if (to >= 0) dst[p * g.ss + to] = v;
+    if (top) dst[p * g.ss + d] = S::empty();
+  }
+  if ((double)bv > LS) {
+    const long long C = ((long long)k * g.fny + j) * g.fnx + i;
+    phi[C] = bv;
+    alpha[C] = S::id(best);
   }
 }
 
@@ -263,26 +279,37 @@ static __global__ void archive_kernel(const int* __restrict__ alpha, int* alpha_
 // Voxel count per grain id over the interior of the argmax map, plus the first
 // (k, j, i)-order index where each id occurs (for the reference's first-seen
 // ordering, QOI.cpp:198-231).  counts[0] = interior cells with no grain.
-// Neighbouring cells mostly share a grain, so the lanes of a warp holding the
-// same id add their count in one atomic from the lowest of them, which also
-// holds their smallest index (a warp's lanes take consecutive interior cells,
-// whose reference-layout indices increase with the lane).
+// A warp takes rows.  Neighbouring cells mostly share a grain, so the lanes of a
+// warp holding the same id add their count in one atomic from the lowest of them,
+// which also holds their smallest index; the cells with no grain (most of a window
+// that is still liquid) are counted in registers, one atomic a warp at its end.
 static __global__ void volume_kernel(const int* __restrict__ alpha, int fnx, int fny, int fnz, int ng,
                               unsigned long long* counts, long long* first) {
-  const long long ni = fnx - 2, nj = fny - 2, nk = fnz - 2;
-  const long long total = ni * nj * nk;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = 1 + idx % ni, j = 1 + (idx / ni) % nj, k = 1 + idx / (ni * nj);
-    const long long C = k * fnx * fny + j * fnx + i;
-    const int a = alpha[C];
-    const int key = (a >= 1 && a <= ng) ? a : 0;
-    const unsigned peers = __match_any_sync(__activemask(), key);
-    if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
-      atomicAdd(counts + key, (unsigned long long)__popc(peers));
-      if (key) atomicMin(first + key, C);
+  const int lane = threadIdx.x & 31, nj = fny - 2;
+  const int nwarps = gridDim.x * (blockDim.x >> 5);
+  const long long rows = (long long)nj * (fnz - 2);
+  unsigned long long none = 0;
+  for (long long r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += nwarps) {
+    const int k = 1 + (int)(r / nj), j = 1 + (int)(r - (long long)(k - 1) * nj);
+    const long long row = ((long long)k * fny + j) * fnx;
+    for (int i0 = 1; i0 < fnx - 1; i0 += 32) {
+      const int i = i0 + lane;
+      const bool on = i < fnx - 1;
+      const int a = on ? alpha[row + i] : 0;
+      const int key = (a >= 1 && a <= ng) ? a : 0;
+      none += on && key == 0;
+      const unsigned grains = __ballot_sync(0xffffffffu, key != 0);
+      if (key) {
+        const unsigned peers = __match_any_sync(grains, key);
+        if (lane == __ffs(peers) - 1) {
+          atomicAdd(counts + key, (unsigned long long)__popc(peers));
+          atomicMin(first + key, row + i);
+        }
+      }
     }
   }
+  for (int o = 16; o > 0; o >>= 1) none += __shfl_down_sync(0xffffffffu, none, o);
+  if (lane == 0 && none) atomicAdd(counts, none);
 }
 
 // Candidate cells of the 3D junction search (QOI3D::searchJunctionsOnImage,
@@ -381,30 +408,52 @@ static __global__ void line_junction_kernel(const int* __restrict__ layers, int 
 //                 diffuse interface integrates |grad phi| to 2 across its width)
 // with central differences of m on the 6 neighbours (halo cells filled first).
 // One partial pair per block; the host adds the partials in block order.
+// A block takes 32 x 8 cell columns over chunks of planes and marches up: every
+// plane's m, with a one-cell rim, is formed once in shared memory (a cell's slots
+// are read 1.4 times in all instead of seven times), three planes at a time.  Chunks
+// of 32 planes, halved down to 2 while the grid has fewer than the launch has blocks.
 template <class S>
-__device__ __forceinline__ float max_phi(const typename S::T* __restrict__ buf, const Grid& g,
-                                         long long d) {
-  float m = S::phi(buf[d]);
-  for (int p = 1; p < g.np; ++p) m = fmaxf(m, S::phi(buf[p * g.ss + d]));
-  return m;
-}
-
-template <class S>
-__global__ void qoi_sums_kernel(const typename S::T* __restrict__ buf, Grid g, double* part) {
-  const long long ni = g.fnx - 2, nj = g.fny - 2, nk = g.fnz - 2;
-  const long long total = ni * nj * nk;
+__global__ void __launch_bounds__(256)
+    qoi_sums_kernel(const typename S::T* __restrict__ buf, Grid g, double* part) {
+  constexpr int W = 34, H = 10;
+  __shared__ float m[3][W * H];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int ntx = (g.fnx - 2 + 31) / 32, nty = (g.fny - 2 + 7) / 8;
+  int np = 32;
+  while (np > 2 && (long long)ntx * nty * ((g.fnz - 2 + np - 1) / np) < gridDim.x) np /= 2;
+  const int nzc = (g.fnz - 2 + np - 1) / np;
   double vol = 0.0, area = 0.0;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int i = 1 + (int)(idx % ni), j = 1 + (int)((idx / ni) % nj), k = 1 + (int)(idx / (ni * nj));
-    const long long d = g.at(i, j, k);
-    const double m = max_phi<S>(buf, g, d);
-    vol += 0.5 * (1.0 + m);
-    const double gx = 0.5 * ((double)max_phi<S>(buf, g, d + 1) - max_phi<S>(buf, g, d - 1));
-    const double gy = 0.5 * ((double)max_phi<S>(buf, g, d + g.xp) - max_phi<S>(buf, g, d - g.xp));
-    const double gz =
-        0.5 * ((double)max_phi<S>(buf, g, d + g.plane()) - max_phi<S>(buf, g, d - g.plane()));
-    area += 0.5 * sqrt(gx * gx + gy * gy + gz * gz);
+  for (int it = blockIdx.x; it < ntx * nty * nzc; it += gridDim.x) {
+    const int x0 = 32 * (it % ntx), y0 = 8 * (it / ntx % nty);  // the rim's first cell
+    const int k0 = 1 + np * (it / (ntx * nty)), k1 = min(k0 + np, g.fnz - 1);
+    auto plane = [&](int k) {
+      for (int c = threadIdx.x; c < W * H; c += 256) {
+        const int i = x0 + c % W, j = y0 + c / W;
+        if (i >= g.fnx || j >= g.fny) continue;
+        const typename S::T* q = buf + g.at(i, j, k);
+        float v = S::phi(q[0]);
+        for (int p = 1; p < g.np; ++p) v = fmaxf(v, S::phi(q[p * g.ss]));
+        m[k % 3][c] = v;
+      }
+    };
+    __syncthreads();  // the previous item's planes have been read
+    plane(k0 - 1);
+    plane(k0);
+    const int i = x0 + 1 + tx, j = y0 + 1 + ty, c = (ty + 1) * W + tx + 1;
+    const bool on = i < g.fnx - 1 && j < g.fny - 1;
+    for (int k = k0; k < k1; ++k) {
+      plane(k + 1);
+      __syncthreads();
+      if (on) {
+        const float* mc = m[k % 3] + c;
+        vol += 0.5 * (1.0 + (double)mc[0]);
+        const double gx = 0.5 * ((double)mc[1] - mc[-1]);
+        const double gy = 0.5 * ((double)mc[W] - mc[-W]);
+        const double gz = 0.5 * ((double)m[(k + 1) % 3][c] - m[(k + 2) % 3][c]);
+        area += 0.5 * sqrt(gx * gx + gy * gy + gz * gz);
+      }
+      __syncthreads();  // plane k - 1 makes room for k + 2
+    }
   }
   __shared__ double rv[256], ra[256];
   rv[threadIdx.x] = vol;

@@ -1099,7 +1099,7 @@ extern "C" cupf_status cupf_apt_move_domain(cupf_apt_handle* h, int32_t* tip_fro
   }
   cupf_status st = fill_halo(h, h->cur);
   if (st) return st;
-  LAUNCH_S(h, layer_sum_kernel, p.fnz, 256, B<S>(h->buf[h->cur]), h->layer_sums, g);
+  LAUNCH_S(h, layer_sum_kernel, p.fnz, kLayerThreads, B<S>(h->buf[h->cur]), h->layer_sums, g);
   CK(cudaGetLastError());
   std::vector<double> sums(p.fnz);
   CK(cudaMemcpyAsync(sums.data(), h->layer_sums, p.fnz * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1136,17 +1136,14 @@ extern "C" cupf_status cupf_apt_move_domain(cupf_apt_handle* h, int32_t* tip_fro
       h->alpha_full = na;
       h->fnz_f = nf;
     }
-    const size_t L = (size_t)g.length();
-    LAUNCH_S(h, collect_kernel, grid_for(L), 256, B<S>(h->buf[h->cur]), h->phi_m, h->alpha_m, g);
+    LAUNCH_S(h, move_layer_kernel, move_layer_blocks(g), 256, B<S>(h->buf[h->cur]),
+             B<S>(h->buf[h->cur ^ 1]), h->phi_m, h->alpha_m, g, swap ? 1 : 0);
     archive_kernel<<<grid_for(plane), 256, 0, h->stream>>>(h->alpha_m, h->alpha_full, h->loss_area,
                                                            p.fnx, p.fny, *move_count, p.num_theta);
-    const long long ni = (long long)(p.fnx - 2) * (p.fny - 2) * (p.fnz - 2) * p.num_pf;
-    LAUNCH_S(h, shift_kernel, grid_for(ni), 256, B<S>(h->buf[h->cur]), B<S>(h->buf[h->cur ^ 1]), g);
     if (swap) {
-      LAUNCH_S(h, copy_halo_kernel, grid_for(halo_cells(g)), 256, B<S>(h->buf[h->cur]),
-               B<S>(h->buf[h->cur ^ 1]), g);
       h->cur ^= 1;
     } else {
+      const long long ni = (long long)(p.fnx - 2) * (p.fny - 2) * (p.fnz - 2) * p.num_pf;
       LAUNCH_S(h, copy_interior_kernel, grid_for(ni), 256, B<S>(h->buf[h->cur ^ 1]),
                B<S>(h->buf[h->cur]), g);
     }

@@ -352,7 +352,7 @@ extern "C" cupf_status cupf_dense_move_domain(cupf_dense_handle* h, int32_t* tip
   }
   cupf_status st = fill_halo(h, h->cur);
   if (st) return st;
-  layer_sum_kernel<DensePhi><<<p.fnz, 256, 0, h->stream>>>(h->buf[h->cur], h->layer_sums, h->g);
+  layer_sum_kernel<DensePhi><<<p.fnz, kLayerThreads, 0, h->stream>>>(h->buf[h->cur], h->layer_sums, h->g);
   CK(cudaGetLastError());
   std::vector<double> sums(p.fnz);
   CK(cudaMemcpyAsync(sums.data(), h->layer_sums, p.fnz * sizeof(double), cudaMemcpyDeviceToHost,
