@@ -403,16 +403,16 @@ static int default_zc(cupf_apt_handle* h) {
 // Work-item shape for a state whose grain ids occupy nz_active interior planes (those
 // within 10 planes of a plane holding an id: the tails the first steps grow).  Quiet
 // items cost next to nothing, so the items that count are the ones the step computes.
-// The lines, measured on line cases on a B200 (us per step, tile height / z chunk):
-//   tile height 4 where it keeps as many warps resident as 8 does (16-bit pairs, and
-//     FP32 but for NUM_PF = 5 and 8), for its finer items: 256x256x512 FP16 768
-//     (4/16) against 841 (8/8), 96^3 FP16 45 (4/2) against 53 (8/1), 117x75x139 FP32
-//     NUM_PF = 6 53 (4/4) against 64 (8/2); where it does not, 8 is faster (192^3 FP32
-//     NUM_PF = 8: 229 against 245), unless the 32x8 tiles leave CTAs without an item
-//     even at one plane each (24x24x32: 8.4 against 16.2);
+// The lines, measured on line cases on a B200 (us per step over steps 51-150, both
+// heights at the chunk the rule gives them):
+//   FP32 takes tile height 4 where it keeps as many warps resident as 8 does (all but
+//     NUM_PF = 5 and 8), for its finer items: 117x75x139 NUM_PF = 6 59 against 65.
+//     16-bit pairs keep 8, whose centre plane is decoded once: 128x128x256 149 against
+//     154, 192^3 240 against 245;
+//   any format takes 4 where the 32x8 tiles would need chunks of one plane to give every
+//     CTA two items: 24x24x32 FP32 14.2 against 16.0;
 //   z chunk: the largest of 16, 8, 4, 2 that gives 2 (tile height 8) or 1.75 (4) items
-//     per resident CTA over the active planes, else 1: within 3 % of the best chunk of
-//     1..32 on those cases and on 128x128x256 and 192^3 FP16.
+//     per resident CTA over the active planes, else 1.
 static cupf_status choose_shape(cupf_apt_handle* h, int nz_active) {
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
@@ -421,7 +421,8 @@ static cupf_status choose_shape(cupf_apt_handle* h, int nz_active) {
   };
   const int r8 = resident_per_sm(h, 8), r4 = resident_per_sm(h, 4);
   if (!h->ty_user) {
-    const int ty = 4 * r4 >= 8 * r8 || tiles(8) * nz_active < (long long)r8 * nsm ? 4 : 8;
+    const bool few = tiles(8) * ((nz_active + 1) / 2) < 2LL * r8 * nsm;
+    const int ty = few || (h->pair_bytes == 8 && 4 * r4 >= 8 * r8) ? 4 : 8;
     if (ty != h->ty) {
       h->ty = ty;
       for (int b = 0; b < 2; ++b)
