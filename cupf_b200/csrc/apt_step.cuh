@@ -73,7 +73,7 @@ struct StepSmem {
   static constexpr bool kDecode = S::kBytes == 4 && TY == 8;
   static constexpr int kDecOff = STAGES * kStageBytes;
   static constexpr int kDecBytes = kDecode ? (NP + 1) * BCELLS * 4 : 0;
-  // per warp: the merged cells' words, merge results and alias words
+  // per warp: its cells' slot-map words, and the merged cells' results and alias words
   static constexpr int kWordOff = kDecOff + kDecBytes;
   static constexpr int kBarOff = kWordOff + TY * (NP + 2) * 32 * 4;
   // + abort word, issued count, item index
@@ -157,6 +157,13 @@ __device__ __forceinline__ void tma_load_plane(void* dst, const CUtensorMap* map
       "l"(map), "r"(x), "r"(y), "r"(z), "r"(0), "r"(smem_u32(bar))
       : "memory");
 }
+
+// Copy one word from global to shared memory without a register (asynchronous; this
+// thread's copies have landed after copy_wait).
+__device__ __forceinline__ void copy_word(uint32_t* dst, const uint32_t* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -307,6 +314,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
   const int m_off = (ty + 1) * BW + 1 +
                     (m_pt == 1 ? -BW : m_pt == 2 ? -1 : m_pt == 4 ? 1 : m_pt == 5 ? BW : 0);
   uint32_t* wbuf = sm.wbuf + ty * ((NP + 2) * 32);
+  uint32_t* wcol = wbuf + lane;  // this cell's words, 32 apart
 
   // the next plane's word 0 and change marks, loaded a plane ahead
   const long long cell0 = (long long)k_begin * plane_pairs + (long long)gy * a.xp + gx;
@@ -327,8 +335,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
   for (int k = k_begin; k < k_end; ++k) {
     const int qk = k - k_begin + 1;
     const long long cell = cell0 + (long long)(k - k_begin) * plane_pairs;
-    uint32_t w[NP];
-    w[0] = next_w0 & kMapCodes;
+    const uint32_t w0 = next_w0 & kMapCodes;
     int n = (int)(next_w0 >> 28);
     // a mark left in redo_out by an earlier step (the item was not computed since)
     // counts too; a neighbour setting it for the next step meanwhile costs only a
@@ -336,9 +343,11 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
     const bool need = valid && (n > NP || next_r0 || next_r1);
     const bool had_mark = next_r0 != 0;
     if (!valid || need) n = 0;
+    // the cell's words into its column of the warp's buffer
+    if (n > 0) wcol[0] = w0;
 #pragma unroll
     for (int j = 1; j < NP; ++j)
-      if (j < n) w[j] = a.map[j * ss + cell];
+      if (j < n) copy_word(wcol + j * 32, a.map + j * ss + cell);
     if (valid && k + 1 < k_end) prefetch(cell + plane_pairs);
     if (plane_T && (qk & 31) == 1) {  // lane l: plane k + l
       float T;
@@ -462,9 +471,6 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
       if (need) {
         const uint32_t info = wbuf[NP * 32 + lane];
         n = (int)(info >> 28);
-#pragma unroll
-        for (int j = 0; j < NP; ++j)
-          if (j < n) w[j] = wbuf[j * 32 + lane];
         uint32_t mark0 = (uint32_t)n;
         if (info & 0x3FFFFu) {
           force_mark = (info >> 16) & 1u;
@@ -475,15 +481,16 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
           }
         }
         if (a.map) {
-          a.map[cell] = (n ? w[0] : 0u) | (mark0 << 28);
+          a.map[cell] = (n ? wcol[0] : 0u) | (mark0 << 28);
 #pragma unroll
           for (int j = 1; j < NP; ++j)
-            if (j < n) a.map[j * ss + cell] = w[j];
+            if (j < n) a.map[j * ss + cell] = wcol[j * 32];
           if (had_mark) a.redo_in[cell] = 0;
         }
       }
       __syncwarp();  // the buffer is rewritten at the next plane
     }
+    copy_wait();
     if (!valid) continue;
 
     P* outp = gout + cell;
@@ -527,7 +534,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
       if (q >= n) break;
-      phc1[q] = __fadd_rn(phi_at(w[q], 3), 1.0f);
+      phc1[q] = __fadd_rn(phi_at(wcol[q * 32], 3), 1.0f);
     }
     if (aliased && map_code(alias, 3) != 0xFu) phc1[0] = __fadd_rn(alias_at(3), 1.0f);
 
@@ -628,9 +635,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
     if (upd) {
 #pragma unroll 1
       for (int j = 0; j < n; ++j) {
-        const P v = update_slot(j, w[0]);
-#pragma unroll
-        for (int q = 0; q + 1 < NP; ++q) w[q] = w[q + 1];
+        const P v = update_slot(j, wcol[j * 32]);
         clive |= !S::is_empty(v);
         put(j, v);
       }
