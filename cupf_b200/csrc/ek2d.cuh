@@ -566,7 +566,9 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
 // two edges and the update formed once: 1 - phi^2 and jat/2 are carried with a row,
 // one reciprocal root per edge serves the normal and the anisotropy's 1/m^2 (the
 // squared gradient is the same before and after the rotation), and the row's Up is
-// formed in FP64 once per row by one lane instead of by every lane.
+// formed in FP64 once per row by one lane instead of by every lane.  Bound by instruction
+// issue: 2048x8192 FP32 181 us per step with the general form, 160 with this one (its 24
+// bytes per cell would take 61), 2048x4096 FP16 102 and 86.
 
 // edge_flux from the sums of the two cells' phi and jat/2 and the difference of
 // their U.
