@@ -711,6 +711,8 @@ __device__ __forceinline__ bool item_quiet(const StepArgs& a, const uint8_t* qui
 // CTAs never touches.  Otherwise each CTA counts itself done once it has drawn past
 // the end; the last one resets both words, so the next launch (or graph replay)
 // starts from zero.
+// Every item is taken only while the error word is clear: after a failed
+// load the steps still queued compute nothing, in launches of either kind.
 struct WorkItems {
   int* work;
   int nitems;
@@ -724,7 +726,9 @@ struct WorkItems {
     if (nitems <= (int)gridDim.x) {  // one item a CTA
       const int it = ticket < nitems ? ticket : -1;
       ticket = nitems;
-      return it;
+      if (it < 0) return it;
+      // one thread's reading decides for the CTA: the word may be set meanwhile
+      return __syncthreads_or(threadIdx.x == 0 && *(volatile const int*)err != 0) ? -1 : it;
     }
     __syncthreads();  // every thread has read the previous index
     if (threadIdx.x == 0) {

@@ -46,6 +46,36 @@ def test_step_wait_bound_runs_out_then_recovers(built):
     assert np.array_equal(ph.view(np.int32), ph2.view(np.int32))
 
 
+@pytest.mark.parametrize("size,z_chunk", [((24, 24, 32), 0), ((48, 40, 56), 0), ((96, 96, 96), 1)],
+                         ids=["one_tile_column", "one_item_a_cta", "items_from_the_counter"])
+def test_steps_after_a_failed_one_compute_nothing(built, size, z_chunk):
+    """The work items of a launch are taken only while no step has failed: what was
+    queued behind a failed step must not run its loads and waits again."""
+    c = cases.line_case(*size, num_pf=5, num_grains=20, seed=2, bc="110")
+    with APTSolver(c) as s:
+        if z_chunk:
+            s.set_tuning(z_chunk)
+        s.init_from_argmax(c.phi, c.alpha)
+        s.set_skip_quiet(False)
+        s.step(2)
+        s.sync()
+        s.active_cells()
+        s.set_wait_limit(1)
+        s.step(1)
+        with pytest.raises(abi.CupfError):
+            s.sync()
+        assert s.active_cells() > 0
+        s.step(50)
+        with pytest.raises(abi.CupfError):
+            s.sync()
+        assert s.active_cells() == 0
+        s.set_wait_limit(0)
+        s.init_from_argmax(c.phi, c.alpha)
+        s.step(1)
+        s.sync()
+        assert s.active_cells() == size[0] * size[1] * size[2]
+
+
 def test_sync_deadline_then_completion(built):
     c = cases.line_case(128, 128, 256, num_pf=8, num_grains=150, seed=0, bc="110")
     with APTSolver(c) as s:
