@@ -433,7 +433,7 @@ static cupf_status choose_shape(cupf_apt_handle* h, int nz_active) {
   int zc = 16;
   while (zc > 1 && tiles(h->ty) * ((nz_active + zc - 1) / zc) < want) zc /= 2;
   set_zc(h, zc);
-  return CUPF_OK;
+  return invalidate_quiet(h);  // the flags are per item
 }
 
 // Interior planes within 10 planes of a plane that holds an id (plane_any[k]
@@ -694,8 +694,8 @@ extern "C" cupf_status cupf_apt_init_from_argmax(cupf_apt_handle* h, const float
 static cupf_status ensure_xfer(cupf_apt_handle* h) {
   if (!h->xfer_ph) {
     const size_t n = (size_t)h->g.length() * h->g.np;
-    CK(cudaMalloc((void**)&h->xfer_ph, n * sizeof(float)));
-    CK(cudaMalloc((void**)&h->xfer_id, n * sizeof(int)));
+    CK(malloc_together({{(void**)&h->xfer_ph, n * sizeof(float)},
+                        {(void**)&h->xfer_id, n * sizeof(int)}}));
   }
   return CUPF_OK;
 }
@@ -710,6 +710,8 @@ extern "C" cupf_status cupf_apt_set_slots(cupf_apt_handle* h, const float* ph, c
   for (size_t i = 0; i < n; ++i)
     if (ids[i] < -1 || ids[i] > id_max)
       return fail(CUPF_ERR_INVALID, "grain id %d at %zu outside [-1, %d]", ids[i], i, id_max);
+  cupf_status st = ensure_xfer(h);  // may fail: before anything of the handle changes
+  if (st) return st;
   if (!h->zc_user) {
     // reference layout: index = i + j*fnx + k*fnx*fny + slot*L
     std::vector<char> plane_any(h->p.fnz, 0);
@@ -722,10 +724,8 @@ extern "C" cupf_status cupf_apt_set_slots(cupf_apt_handle* h, const float* ph, c
               plane_any[k] = 1;
               break;
             }
-    if (cupf_status cs = choose_shape(h, active_planes(plane_any, h->p.fnz))) return cs;
+    if ((st = choose_shape(h, active_planes(plane_any, h->p.fnz)))) return st;
   }
-  cupf_status st = ensure_xfer(h);
-  if (st) return st;
   CK(cudaMemcpyAsync(h->xfer_ph, ph, n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->xfer_id, ids, n * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   LAUNCH_S(h, import_kernel, grid_for(n), 256, B<S>(h->buf[0]), h->xfer_ph, h->xfer_id, h->g);
@@ -916,10 +916,9 @@ extern "C" cupf_status cupf_apt_grain_volumes(cupf_apt_handle* h, int32_t num_gr
   if (h->counts_cap < num_grains + 1) {
     if (h->counts) cudaFree(h->counts);
     if (h->first) cudaFree(h->first);
-    h->counts = nullptr;
-    h->first = nullptr;
-    CK(cudaMalloc((void**)&h->counts, (num_grains + 1) * sizeof(unsigned long long)));
-    CK(cudaMalloc((void**)&h->first, (num_grains + 1) * sizeof(long long)));
+    h->counts_cap = 0;
+    CK(malloc_together({{(void**)&h->counts, (num_grains + 1) * sizeof(unsigned long long)},
+                        {(void**)&h->first, (num_grains + 1) * sizeof(long long)}}));
     h->counts_cap = num_grains + 1;
   }
   CK(cudaMemsetAsync(h->counts, 0, (num_grains + 1) * sizeof(unsigned long long), h->stream));
@@ -1034,9 +1033,9 @@ extern "C" cupf_status cupf_apt_nucl_init(cupf_apt_handle* h) {
   const long long nc = (long long)h->cnx * h->cny * h->cnz;
   if (nc < 1) return fail(CUPF_ERR_INVALID, "grid smaller than one nucleation cell");
   if (!h->nucl_status) {
-    CK(cudaMalloc((void**)&h->nucl_status, nc * sizeof(int)));
-    CK(cudaMalloc((void**)&h->nucl_count, sizeof(int)));
-    CK(cudaMalloc((void**)&h->nucl_sphere, (size_t)w * w * w * sizeof(float)));
+    CK(malloc_together({{(void**)&h->nucl_status, nc * sizeof(int)},
+                        {(void**)&h->nucl_count, sizeof(int)},
+                        {(void**)&h->nucl_sphere, (size_t)w * w * w * sizeof(float)}}));
   }
   // nucleus profile (add_nucl :515-528): tanh(dx*((1+pts)/2 - |offset|) / sqrt2)
   std::vector<float> sph((size_t)w * w * w);
@@ -1092,10 +1091,10 @@ extern "C" cupf_status cupf_apt_move_domain(cupf_apt_handle* h, int32_t* tip_fro
   const cupf_apt_params& p = h->p;
   if (!h->alpha_full) {
     h->fnz_f = p.fnz * 4 + 8;  // archive capacity in layers; grown on demand below
-    CK(cudaMalloc((void**)&h->alpha_full, (size_t)p.fnx * p.fny * h->fnz_f * sizeof(int)));
+    CK(malloc_together({{(void**)&h->alpha_full, (size_t)p.fnx * p.fny * h->fnz_f * sizeof(int)},
+                        {(void**)&h->loss_area, p.num_theta * sizeof(int)}}));
     CK(cudaMemsetAsync(h->alpha_full, 0, (size_t)p.fnx * p.fny * h->fnz_f * sizeof(int),
                        h->stream));
-    CK(cudaMalloc((void**)&h->loss_area, p.num_theta * sizeof(int)));
     CK(cudaMemsetAsync(h->loss_area, 0, p.num_theta * sizeof(int), h->stream));
   }
   cupf_status st = fill_halo(h, h->cur);
@@ -1124,19 +1123,21 @@ extern "C" cupf_status cupf_apt_move_domain(cupf_apt_handle* h, int32_t* tip_fro
   // which must then hold the moved state: there the copy back stays.
   const int cur0 = h->cur;
   const bool swap = p.thermalType != 3 && p.thermalType != 4;
+  // grow the archive for every layer to be moved, before the first one is
+  int nf = h->fnz_f;
+  while (*tip_front >= tip_thres && *move_count + (*tip_front - tip_thres + 1) + 1 > nf) nf *= 2;
+  if (nf > h->fnz_f) {
+    int* na = nullptr;
+    CK(malloc_together({{(void**)&na, (size_t)plane * nf * sizeof(int)}}));
+    CK(cudaMemsetAsync(na, 0, (size_t)plane * nf * sizeof(int), h->stream));
+    CK(cudaMemcpyAsync(na, h->alpha_full, (size_t)plane * h->fnz_f * sizeof(int),
+                       cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    cudaFree(h->alpha_full);
+    h->alpha_full = na;
+    h->fnz_f = nf;
+  }
   while (*tip_front >= tip_thres) {
-    if (*move_count + 2 > h->fnz_f) {  // grow the archive
-      const int nf = h->fnz_f * 2;
-      int* na = nullptr;
-      CK(cudaMalloc((void**)&na, (size_t)plane * nf * sizeof(int)));
-      CK(cudaMemsetAsync(na, 0, (size_t)plane * nf * sizeof(int), h->stream));
-      CK(cudaMemcpyAsync(na, h->alpha_full, (size_t)plane * h->fnz_f * sizeof(int),
-                         cudaMemcpyDeviceToDevice, h->stream));
-      CK(cudaStreamSynchronize(h->stream));
-      cudaFree(h->alpha_full);
-      h->alpha_full = na;
-      h->fnz_f = nf;
-    }
     LAUNCH_S(h, move_layer_kernel, move_layer_blocks(g), 256, B<S>(h->buf[h->cur]),
              B<S>(h->buf[h->cur ^ 1]), h->phi_m, h->alpha_m, g, swap ? 1 : 0);
     archive_kernel<<<grid_for(plane), 256, 0, h->stream>>>(h->alpha_m, h->alpha_full, h->loss_area,

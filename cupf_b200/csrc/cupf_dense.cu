@@ -345,9 +345,9 @@ extern "C" cupf_status cupf_dense_move_domain(cupf_dense_handle* h, int32_t* tip
   const long long plane = (long long)p.fnx * p.fny;
   if (!h->alpha_full) {
     h->fnz_f = p.fnz * 4 + 8;
-    CK(cudaMalloc((void**)&h->alpha_full, (size_t)plane * h->fnz_f * sizeof(int)));
+    CK(malloc_together({{(void**)&h->alpha_full, (size_t)plane * h->fnz_f * sizeof(int)},
+                        {(void**)&h->loss_area, p.num_theta * sizeof(int)}}));
     CK(cudaMemsetAsync(h->alpha_full, 0, (size_t)plane * h->fnz_f * sizeof(int), h->stream));
-    CK(cudaMalloc((void**)&h->loss_area, p.num_theta * sizeof(int)));
     CK(cudaMemsetAsync(h->loss_area, 0, p.num_theta * sizeof(int), h->stream));
   }
   cupf_status st = fill_halo(h, h->cur);

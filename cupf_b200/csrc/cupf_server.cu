@@ -481,8 +481,9 @@ static cupf_status retire(cupf_server* s, Request* r, int cur) {
   if (s->counts_cap < ng + 1) {
     if (s->d_counts) cudaFree(s->d_counts);
     if (s->d_first) cudaFree(s->d_first);
-    CK(cudaMalloc((void**)&s->d_counts, (ng + 1) * sizeof(unsigned long long)));
-    CK(cudaMalloc((void**)&s->d_first, (ng + 1) * sizeof(long long)));
+    s->counts_cap = 0;
+    CK(malloc_together({{(void**)&s->d_counts, (ng + 1) * sizeof(unsigned long long)},
+                        {(void**)&s->d_first, (ng + 1) * sizeof(long long)}}));
     s->counts_cap = ng + 1;
   }
   CK(cudaMemsetAsync(s->d_counts, 0, (ng + 1) * sizeof(unsigned long long), st));
@@ -563,8 +564,10 @@ static cupf_status rebuild(cupf_server* s) {
   s->nitems = (int)items.size();
   if (s->nitems > s->items_cap) {
     if (s->d_items) cudaFree(s->d_items);
-    s->items_cap = std::max(s->nitems, 2 * s->items_cap);
-    CK(cudaMalloc((void**)&s->d_items, s->items_cap * sizeof(int4)));
+    const int cap = std::max(s->nitems, 2 * s->items_cap);
+    s->items_cap = 0;
+    CK(malloc_together({{(void**)&s->d_items, cap * sizeof(int4)}}));
+    s->items_cap = cap;
   }
   if (s->nitems)
     CK(cudaMemcpyAsync(s->d_items, items.data(), items.size() * sizeof(int4),
