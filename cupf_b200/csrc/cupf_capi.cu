@@ -13,6 +13,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -98,7 +99,8 @@ struct cupf_apt_handle {
   uint8_t* quiet[2] = {nullptr, nullptr};
   size_t quiet_cap = 0;
   // slot maps of the step and their change marks per buffer (StepArgs::map,
-  // redo_in/out); NULL where the device had no room for them
+  // redo_in/out); NULL where the device has no room for them (alloc_maps)
+  std::recursive_timed_mutex map_use;  // held by the calls that use them
   uint32_t* map = nullptr;
   uint8_t* redo[2] = {nullptr, nullptr};
   bool skip_quiet = true;
@@ -141,7 +143,7 @@ static const char* kOk = "";
 
 static cupf_status upload(float** dst, const float* src, size_t n, cudaStream_t s) {
   if (n == 0) n = 1;
-  CK(cudaMalloc((void**)dst, n * sizeof(float)));
+  CK(device_malloc(dst, n * sizeof(float)));
   if (src)
     CK(cudaMemcpyAsync(*dst, src, n * sizeof(float), cudaMemcpyHostToDevice, s));
   else
@@ -198,8 +200,11 @@ static cupf_status make_tmap(cupf_apt_handle* h, int b) {
   });
 }
 
+static void forget_map_owner(cupf_apt_handle* h);
+
 static void free_handle(cupf_apt_handle* h) {
   if (!h) return;
+  forget_map_owner(h);
   cudaSetDevice(h->device);
   void* ptrs[] = {h->buf[0], h->buf[1], h->x, h->y, h->z, h->sint, h->cost, h->orient, h->X_mac, h->Y_mac,
                   h->Z_mac, h->t_mac, h->psi_mac, h->T_3D, h->phi_m, h->alpha_m, h->err, h->work,
@@ -344,23 +349,63 @@ static cupf_status invalidate_maps(cupf_apt_handle* h) {
   return CUPF_OK;
 }
 
-// Slot maps and change marks of the step (a quarter of the FP32 pair buffers'
-// size).  A grid whose pairs leave no room for them runs without: every cell is
-// then merged every step, with the same results.
+// Left free beside the slot maps: for what the process allocates outside this library
+// and for the driver (kernels load their code when first launched).
+constexpr size_t kMapReserve = (size_t)2 << 30;
+
+// The handles that hold slot maps.  Whoever works with a handle's maps holds its
+// map_use; a release takes that lock only for a bounded time, so two calls that want
+// each other's maps end with one of them refused.
+static std::mutex g_map_mutex;
+static std::vector<cupf_apt_handle*> g_map_owners;
+
+static void free_maps(cupf_apt_handle* h) {
+  for (void* p : {(void*)h->map, (void*)h->redo[0], (void*)h->redo[1]})
+    if (p) cudaFree(p);
+  h->map = nullptr;
+  h->redo[0] = h->redo[1] = nullptr;
+}
+
+static void forget_map_owner(cupf_apt_handle* h) {
+  std::lock_guard<std::mutex> lock(g_map_mutex);
+  g_map_owners.erase(std::remove(g_map_owners.begin(), g_map_owners.end(), h), g_map_owners.end());
+}
+
+bool release_slot_maps() {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(g_map_mutex);
+  for (size_t i = 0; i < g_map_owners.size(); ++i) {
+    cupf_apt_handle* h = g_map_owners[i];
+    if (h->device != device) continue;
+    std::unique_lock<std::recursive_timed_mutex> use(h->map_use, std::chrono::seconds(1));
+    if (!use || cudaStreamSynchronize(h->stream) != cudaSuccess) continue;
+    free_maps(h);
+    g_map_owners.erase(g_map_owners.begin() + i);
+    return true;
+  }
+  return false;
+}
+
+// Slot maps and change marks of the step (a quarter of the FP32 pair buffers' size).
+// A grid whose pairs leave no room for them runs without, and they are given back
+// when any other allocation of the library needs the room (release_slot_maps): every
+// cell is then merged every step, with the same results.
 static cupf_status alloc_maps(cupf_apt_handle* h) {
   const size_t cells = (size_t)h->g.ss;
-  if (cudaMalloc((void**)&h->map, cells * h->g.np * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc((void**)&h->redo[0], cells) != cudaSuccess ||
-      cudaMalloc((void**)&h->redo[1], cells) != cudaSuccess) {
-    cudaGetLastError();  // not an error of the call
-    for (void* p : {(void*)h->map, (void*)h->redo[0], (void*)h->redo[1]})
-      if (p) cudaFree(p);
-    h->map = nullptr;
-    h->redo[0] = h->redo[1] = nullptr;
+  const size_t bytes = cells * (h->g.np * sizeof(uint32_t) + 2);
+  size_t room = ~(size_t)0, total = 0;
+  if (bytes > kMapReserve / 64) CK(cudaMemGetInfo(&room, &total));  // the query takes 80 us
+  if (room - bytes < kMapReserve || room < bytes ||
+      malloc_together({{(void**)&h->map, cells * h->g.np * sizeof(uint32_t)},
+                       {(void**)&h->redo[0], cells},
+                       {(void**)&h->redo[1], cells}}, false) != cudaSuccess)
     return CUPF_OK;
-  }
   for (int b = 0; b < 2; ++b) CK(cudaMemsetAsync(h->redo[b], 0, cells, h->stream));
-  return invalidate_maps(h);
+  if (cupf_status st = invalidate_maps(h)) return st;
+  std::lock_guard<std::mutex> lock(g_map_mutex);
+  g_map_owners.push_back(h);
+  return CUPF_OK;
 }
 
 // Resident CTAs per SM the step kernel is compiled for (step_min_blocks).
@@ -522,7 +567,7 @@ extern "C" cupf_status cupf_apt_create(const cupf_apt_params* p, const cupf_apt_
   TRY(cuda(cudaEventCreate(&h->ev1), "event"));
   const size_t bbytes = (size_t)h->g.ss * h->g.np * h->pair_bytes;
   for (int b = 0; b < 2; ++b) {
-    TRY(cuda(cudaMalloc((void**)&h->buf[b], bbytes), "slot buffer"));
+    TRY(cuda(device_malloc(&h->buf[b], bbytes), "slot buffer"));
     TRY(cuda(cudaMemsetAsync(h->buf[b], 0xFF, bbytes, h->stream), "memset"));
   }
   const int nth = 2 * p->num_theta + 1;
@@ -531,7 +576,7 @@ extern "C" cupf_status cupf_apt_create(const cupf_apt_params* p, const cupf_apt_
   TRY(upload(&h->z, in->z, p->fnz, h->stream));
   h->z_host.assign(in->z, in->z + p->fnz);
   h->z64_host.assign(in->z, in->z + p->fnz);
-  TRY(cuda(cudaMalloc((void**)&h->z64, p->fnz * sizeof(double)), "z64"));
+  TRY(cuda(device_malloc(&h->z64, p->fnz * sizeof(double)), "z64"));
   TRY(cuda(cudaMemcpyAsync(h->z64, h->z64_host.data(), p->fnz * sizeof(double),
                            cudaMemcpyHostToDevice, h->stream), "z64 upload"));
   TRY(upload(&h->sint, in->sint, nth, h->stream));
@@ -551,25 +596,25 @@ extern "C" cupf_status cupf_apt_create(const cupf_apt_params* p, const cupf_apt_
   TRY(upload(&h->T_3D, in->T_3D, in->T_3D ? mNx * mNy * mNz * mNt : 16, h->stream));
   h->has_T3D = in->T_3D != nullptr;
   const size_t L = (size_t)h->g.length();
-  TRY(cuda(cudaMalloc((void**)&h->phi_m, L * sizeof(float)), "phi"));
-  TRY(cuda(cudaMalloc((void**)&h->alpha_m, L * sizeof(int)), "alpha"));
+  TRY(cuda(device_malloc(&h->phi_m, L * sizeof(float)), "phi"));
+  TRY(cuda(device_malloc(&h->alpha_m, L * sizeof(int)), "alpha"));
   TRY(cuda(cudaMemsetAsync(h->phi_m, 0, L * sizeof(float), h->stream), "memset"));
   TRY(cuda(cudaMemsetAsync(h->alpha_m, 0, L * sizeof(int), h->stream), "memset"));
-  TRY(cuda(cudaMalloc((void**)&h->err, sizeof(int)), "err"));
+  TRY(cuda(device_malloc(&h->err, sizeof(int)), "err"));
   TRY(cuda(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "memset"));
-  TRY(cuda(cudaMalloc((void**)&h->work, 2 * sizeof(int)), "work"));
+  TRY(cuda(device_malloc(&h->work, 2 * sizeof(int)), "work"));
   TRY(cuda(cudaMemsetAsync(h->work, 0, 2 * sizeof(int), h->stream), "memset"));
   // flags for the most items any tile height gives (32x4 tiles, z chunks of 1)
   h->quiet_cap = (size_t)((p->fnx - 2 + TX - 1) / TX) * ((p->fny - 2 + 4 - 1) / 4) * (p->fnz - 2);
   for (int b = 0; b < 2; ++b) {
-    TRY(cuda(cudaMalloc((void**)&h->quiet[b], h->quiet_cap), "quiet flags"));
+    TRY(cuda(device_malloc(&h->quiet[b], h->quiet_cap), "quiet flags"));
     TRY(cuda(cudaMemsetAsync(h->quiet[b], 0, h->quiet_cap, h->stream), "memset"));
   }
-  TRY(cuda(cudaMalloc((void**)&h->active_cells, sizeof(unsigned long long)), "counter"));
+  TRY(cuda(device_malloc(&h->active_cells, sizeof(unsigned long long)), "counter"));
   TRY(cuda(cudaMemsetAsync(h->active_cells, 0, sizeof(unsigned long long), h->stream), "memset"));
-  TRY(cuda(cudaMalloc((void**)&h->overflows, 2 * sizeof(unsigned long long)), "counter"));
+  TRY(cuda(device_malloc(&h->overflows, 2 * sizeof(unsigned long long)), "counter"));
   TRY(cuda(cudaMemsetAsync(h->overflows, 0, 2 * sizeof(unsigned long long), h->stream), "memset"));
-  TRY(cuda(cudaMalloc((void**)&h->layer_sums, p->fnz * sizeof(double)), "layer sums"));
+  TRY(cuda(device_malloc(&h->layer_sums, p->fnz * sizeof(double)), "layer sums"));
   for (int b = 0; b < 2; ++b) TRY(make_tmap(h, b));
   TRY(alloc_maps(h));  // last: takes only room the rest left
   const char* zc_env = getenv("CUPF_ZC");
@@ -656,6 +701,7 @@ static cupf_status fill_halo(cupf_apt_handle* h, int b);
 extern "C" cupf_status cupf_apt_init_from_argmax(cupf_apt_handle* h, const float* phi,
                                                  const int32_t* alpha) {
   if (!h || !phi || !alpha) return fail(CUPF_ERR_INVALID, "null argument");
+  std::lock_guard<std::recursive_timed_mutex> use(h->map_use);
   CK(cudaSetDevice(h->device));
   const size_t L = (size_t)h->g.length();
   const int id_max = h->prec == CUPF_PREC_FP32 ? 0x7FFFFFFF : 32767;
@@ -703,6 +749,7 @@ static cupf_status ensure_xfer(cupf_apt_handle* h) {
 extern "C" cupf_status cupf_apt_set_slots(cupf_apt_handle* h, const float* ph, const int32_t* ids,
                                           int64_t steps_done) {
   if (!h || !ph || !ids) return fail(CUPF_ERR_INVALID, "null argument");
+  std::lock_guard<std::recursive_timed_mutex> use(h->map_use);
   CK(cudaSetDevice(h->device));
   const size_t L = (size_t)h->g.length();
   const size_t n = L * h->g.np;
@@ -774,6 +821,7 @@ extern "C" cupf_status cupf_apt_step(cupf_apt_handle* h, int32_t nsteps,
   if (!h) return fail(CUPF_ERR_INVALID, "null handle");
   if (!h->initialised) return fail(CUPF_ERR_STATE, "step before init");
   if (nsteps < 0) return fail(CUPF_ERR_INVALID, "nsteps < 0");
+  std::lock_guard<std::recursive_timed_mutex> use(h->map_use);
   CK(cudaSetDevice(h->device));
   for (int n = 0; n < nsteps; ++n) {
     // t of step m (1-based): (float)m * dt * tau0, as (2*kt+1)*dt*tau0 in evolve
@@ -840,11 +888,11 @@ extern "C" cupf_status cupf_apt_junction_candidates(cupf_apt_handle* h, int64_t*
     if (h->jcand) cudaFree(h->jcand);
     h->jcand = nullptr;
     h->jcand_cap = 0;
-    CK(cudaMalloc((void**)&h->jcand, want * sizeof(long long)));
+    CK(device_malloc(&h->jcand, want * sizeof(long long)));
     h->jcand_cap = want;
   }
-  if (!h->jcount) CK(cudaMalloc((void**)&h->jcount, sizeof(unsigned long long)));
-  if (!h->jdistinct) CK(cudaMalloc((void**)&h->jdistinct, (size_t)ni));
+  if (!h->jcount) CK(device_malloc(&h->jcount, sizeof(unsigned long long)));
+  if (!h->jdistinct) CK(device_malloc(&h->jdistinct, (size_t)ni));
   CK(cudaMemsetAsync(h->jcount, 0, sizeof(unsigned long long), h->stream));
   junction_candidates_kernel<<<grid_for(ni), 256, 0, h->stream>>>(
       h->alpha_m, g.fnx, g.fny, g.fnz, h->jcand, cap, h->jcount, h->jdistinct);
@@ -881,9 +929,9 @@ extern "C" cupf_status cupf_line_junction_candidates(int32_t device, int32_t fnx
   int32_t* d_layers = nullptr;
   long long* d_out = nullptr;
   unsigned long long* d_count = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&d_layers, lbytes, st);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_out, want * sizeof(long long), st);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&d_count, sizeof(unsigned long long), st);
+  cudaError_t e = with_room([&] { return cudaMallocAsync((void**)&d_layers, lbytes, st); });
+  if (e == cudaSuccess) e = with_room([&] { return cudaMallocAsync((void**)&d_out, want * sizeof(long long), st); });
+  if (e == cudaSuccess) e = with_room([&] { return cudaMallocAsync((void**)&d_count, sizeof(unsigned long long), st); });
   unsigned long long n = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_layers, layers, lbytes, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st);
@@ -940,7 +988,7 @@ extern "C" cupf_status cupf_apt_qoi_sums(cupf_apt_handle* h, double* out) {
   if (!h->initialised) return fail(CUPF_ERR_STATE, "state not initialised");
   CK(cudaSetDevice(h->device));
   const int nb = 148 * 4;
-  if (!h->qoi_part) CK(cudaMalloc((void**)&h->qoi_part, 2 * nb * sizeof(double)));
+  if (!h->qoi_part) CK(device_malloc(&h->qoi_part, 2 * nb * sizeof(double)));
   cupf_status st = fill_halo(h, h->cur);
   if (st) return st;
   LAUNCH_S(h, qoi_sums_kernel, nb, 256, B<S>(h->buf[h->cur]), h->g, h->qoi_part);
@@ -1067,6 +1115,7 @@ extern "C" cupf_status cupf_apt_nucl_reset(cupf_apt_handle* h) {
 extern "C" cupf_status cupf_apt_nucleate(cupf_apt_handle* h, int32_t use_initial_undercooling,
                                          int32_t* total) {
   if (!h || !h->nucl_status) return fail(CUPF_ERR_STATE, "nucleation not initialised");
+  std::lock_guard<std::recursive_timed_mutex> use(h->map_use);
   CK(cudaSetDevice(h->device));
   const long long nc = (long long)h->cnx * h->cny * h->cnz;
   NuclArgs a = nucl_args(h, use_initial_undercooling);
@@ -1086,6 +1135,7 @@ extern "C" cupf_status cupf_apt_move_domain(cupf_apt_handle* h, int32_t* tip_fro
                                             int32_t* moved) {
   if (!h || !tip_front || !move_count || !moved) return fail(CUPF_ERR_INVALID, "null argument");
   if (!h->initialised) return fail(CUPF_ERR_STATE, "state not initialised");
+  std::lock_guard<std::recursive_timed_mutex> use(h->map_use);
   CK(cudaSetDevice(h->device));
   const Grid& g = h->g;
   const cupf_apt_params& p = h->p;

@@ -72,7 +72,7 @@ void free_handle(cupf_dense_handle* h) {
 }
 
 cupf_status upload(float** dst, const float* src, size_t n, cudaStream_t s) {
-  CK(cudaMalloc((void**)dst, std::max<size_t>(n, 1) * sizeof(float)));
+  CK(device_malloc(dst, std::max<size_t>(n, 1) * sizeof(float)));
   if (n) CK(cudaMemcpyAsync(*dst, src, n * sizeof(float), cudaMemcpyHostToDevice, s));
   return CUPF_OK;
 }
@@ -195,16 +195,16 @@ extern "C" cupf_status cupf_dense_create(const cupf_apt_params* p, const cupf_ap
   TRY(cuda(cudaEventCreate(&h->ev0), "event"));
   TRY(cuda(cudaEventCreate(&h->ev1), "event"));
   const size_t fbytes = (size_t)h->len * h->np * sizeof(float);
-  for (int b = 0; b < 2; ++b) TRY(cuda(cudaMalloc((void**)&h->buf[b], fbytes), "phi buffer"));
+  for (int b = 0; b < 2; ++b) TRY(cuda(device_malloc(&h->buf[b], fbytes), "phi buffer"));
   for (int b = 0; b < 2; ++b) {
-    TRY(cuda(cudaMalloc((void**)&h->cnt[b], h->len * sizeof(int)), "list counts"));
+    TRY(cuda(device_malloc(&h->cnt[b], h->len * sizeof(int)), "list counts"));
     TRY(cuda(cudaMemsetAsync(h->cnt[b], 0, h->len * sizeof(int), h->stream), "memset"));
-    TRY(cuda(cudaMalloc((void**)&h->lid[b], (size_t)kDenseListMax * h->len * sizeof(unsigned short)),
+    TRY(cuda(device_malloc(&h->lid[b], (size_t)kDenseListMax * h->len * sizeof(unsigned short)),
              "lists"));
-    TRY(cuda(cudaMalloc((void**)&h->lval[b], (size_t)kDenseListMax * h->len * sizeof(float)),
+    TRY(cuda(device_malloc(&h->lval[b], (size_t)kDenseListMax * h->len * sizeof(float)),
              "lists"));
   }
-  TRY(cuda(cudaMalloc((void**)&h->overflow, 2 * sizeof(unsigned long long)), "overflow counter"));
+  TRY(cuda(device_malloc(&h->overflow, 2 * sizeof(unsigned long long)), "overflow counter"));
   TRY(cuda(cudaMemsetAsync(h->overflow, 0, 2 * sizeof(unsigned long long), h->stream), "memset"));
   if (in->x) TRY(upload(&h->x, in->x, p->fnx, h->stream));
   if (in->y) TRY(upload(&h->y, in->y, p->fny, h->stream));
@@ -215,11 +215,11 @@ extern "C" cupf_status cupf_dense_create(const cupf_apt_params* p, const cupf_ap
     pack_orientations(in->sint, in->cost, p->num_theta, ot.data());
     TRY(upload(&h->orient, ot.data(), ot.size(), h->stream));
   }
-  TRY(cuda(cudaMalloc((void**)&h->phi_m, h->len * sizeof(float)), "phi field"));
-  TRY(cuda(cudaMalloc((void**)&h->alpha_m, h->len * sizeof(int)), "alpha field"));
-  TRY(cuda(cudaMalloc((void**)&h->argmax, h->len * sizeof(int)), "argmax"));
+  TRY(cuda(device_malloc(&h->phi_m, h->len * sizeof(float)), "phi field"));
+  TRY(cuda(device_malloc(&h->alpha_m, h->len * sizeof(int)), "alpha field"));
+  TRY(cuda(device_malloc(&h->argmax, h->len * sizeof(int)), "argmax"));
   TRY(cuda(cudaMemsetAsync(h->argmax, 0, h->len * sizeof(int), h->stream), "memset"));
-  TRY(cuda(cudaMalloc((void**)&h->layer_sums, p->fnz * sizeof(double)), "layer sums"));
+  TRY(cuda(device_malloc(&h->layer_sums, p->fnz * sizeof(double)), "layer sums"));
   TRY(cuda(cudaStreamSynchronize(h->stream), "sync"));
   *out = h;
   return CUPF_OK;
@@ -243,7 +243,7 @@ extern "C" cupf_status cupf_dense_init_from_argmax(cupf_dense_handle* h, const f
       if (p) cudaFree(p);
     }
   } stage;
-  CK(cudaMalloc((void**)&stage.p, h->len * sizeof(float)));
+  CK(device_malloc(&stage.p, h->len * sizeof(float)));
   CK(cudaMemcpyAsync(stage.p, phi, h->len * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->alpha_m, alpha, h->len * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   dense_init_kernel<<<grid_for(h->len), 256, 0, h->stream>>>(h->buf[0], h->buf[1], stage.p,
@@ -369,7 +369,7 @@ extern "C" cupf_status cupf_dense_move_domain(cupf_dense_handle* h, int32_t* tip
     if (*move_count + 2 > h->fnz_f) {  // grow the archive
       const int nf = h->fnz_f * 2;
       int* na = nullptr;
-      CK(cudaMalloc((void**)&na, (size_t)plane * nf * sizeof(int)));
+      CK(device_malloc(&na, (size_t)plane * nf * sizeof(int)));
       CK(cudaMemsetAsync(na, 0, (size_t)plane * nf * sizeof(int), h->stream));
       CK(cudaMemcpyAsync(na, h->alpha_full, (size_t)plane * h->fnz_f * sizeof(int),
                          cudaMemcpyDeviceToDevice, h->stream));

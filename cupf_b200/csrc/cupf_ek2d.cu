@@ -216,9 +216,9 @@ extern "C" cupf_status cupf_ek2d_create(const cupf_ek2d_params* p, int32_t preci
   cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
-  for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = cudaMalloc(&h->buf[b], 3 * h->plane * h->vbytes);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->stage, 4 * (size_t)h->fnx * h->fny * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&h->d_rows, h->fny * sizeof(double));
+  for (int b = 0; b < 2 && e == cudaSuccess; ++b) e = device_malloc(&h->buf[b], 3 * h->plane * h->vbytes);
+  if (e == cudaSuccess) e = device_malloc(&h->stage, 4 * (size_t)h->fnx * h->fny * sizeof(float));
+  if (e == cudaSuccess) e = device_malloc(&h->d_rows, h->fny * sizeof(double));
   for (int b = 0; b < 2 && e == cudaSuccess; ++b)
     e = cudaMemsetAsync(h->buf[b], 0, 3 * h->plane * h->vbytes, h->stream);
   if (e != cudaSuccess)
@@ -365,7 +365,7 @@ extern "C" cupf_status cupf_ek2d_get_state_f64(cupf_ek2d_handle* h, double* psi,
   CK(cudaSetDevice(h->device));
   const size_t n = (size_t)h->fnx * h->fny;
   double* d = nullptr;
-  CK(cudaMalloc((void**)&d, 4 * n * sizeof(double)));
+  CK(device_malloc(&d, 4 * n * sizeof(double)));
   double* part[4] = {d, d + n, d + 2 * n, d + 3 * n};
   cupf_status st = with_ek_storage(h->prec, [&](auto tag) -> cupf_status {
     using S = decltype(tag);

@@ -666,14 +666,14 @@ extern "C" cupf_status cupf_server_create(const cupf_server_config* cfg, cupf_se
   CK(cudaEventCreate(&s->ev_round[0]));
   CK(cudaEventCreate(&s->ev_round[1]));
   s->slots.assign(cfg->max_active, 0);
-  CK(cudaMalloc((void**)&s->d_sims, cfg->max_active * sizeof(BatchSim)));
+  CK(device_malloc(&s->d_sims, cfg->max_active * sizeof(BatchSim)));
   CK(cudaMemset(s->d_sims, 0, cfg->max_active * sizeof(BatchSim)));
-  CK(cudaMalloc((void**)&s->d_tmaps, 2 * cfg->max_active * sizeof(CUtensorMap)));
-  CK(cudaMalloc((void**)&s->d_next, 4 * sizeof(int)));  // a work counter pair per tile height
+  CK(device_malloc(&s->d_tmaps, 2 * cfg->max_active * sizeof(CUtensorMap)));
+  CK(device_malloc(&s->d_next, 4 * sizeof(int)));  // a work counter pair per tile height
   CK(cudaMemset(s->d_next, 0, 4 * sizeof(int)));
-  CK(cudaMalloc((void**)&s->d_err, sizeof(int)));
+  CK(device_malloc(&s->d_err, sizeof(int)));
   CK(cudaMemset(s->d_err, 0, sizeof(int)));
-  CK(cudaMalloc((void**)&s->d_part, 2 * 148 * 4 * sizeof(double)));
+  CK(device_malloc(&s->d_part, 2 * 148 * 4 * sizeof(double)));
   size_t fr = 0, tot = 0;
   CK(cudaMemGetInfo(&fr, &tot));
   const size_t reserve = (size_t)2 << 30;

@@ -117,7 +117,10 @@ size_t cupf_struct_size(int which);
 
 /* Allocate device state and upload parameters and thermal inputs.
  * Replaces APTPhaseField::cudaSetup (3DgrainMPI/APTPhaseField.cu:569-637).
- * device: CUDA ordinal.  precision: storage type of the phi slots. */
+ * device: CUDA ordinal.  precision: storage type of the phi slots.
+ * Where enough of the device stays free beside it, the handle also takes optional memory
+ * (4 * num_pf + 2 bytes per cell) that saves the step work; any allocation of this
+ * library that finds no room gets it back, with the same results afterwards. */
 cupf_status cupf_apt_create(const cupf_apt_params* p, const cupf_apt_inputs* in,
                             int device, cupf_precision precision,
                             cupf_apt_handle** out);

@@ -1,6 +1,6 @@
 /* Stand-in for a device with little memory: loaded with LD_PRELOAD before the CUDA
  * runtime, it refuses device allocations on the host and passes the others on.
- * alloc_fail_next(n): after n more allocations, refuse one.
+ * alloc_refuse_from(n): after n more allocations, refuse every one (-1: none).
  * alloc_limit(bytes): refuse what would take the live total past the limit (0: none).
  * alloc_live(): bytes held now.  alloc_refused(): allocations refused so far. */
 #define _GNU_SOURCE
@@ -10,11 +10,11 @@
 
 enum { kOk = 0, kOutOfMemory = 2, kTable = 1 << 16 };
 static pthread_mutex_t lock = PTHREAD_MUTEX_INITIALIZER;
-static long fail_next = -1, refused = 0;
+static long granted = -1, refused = 0;
 static size_t limit = 0, live = 0;
 static struct { void* p; size_t n; } held[kTable];
 
-void alloc_fail_next(long n) { fail_next = n; }
+void alloc_refuse_from(long n) { granted = n; }
 void alloc_limit(size_t bytes) { limit = bytes; }
 size_t alloc_live(void) { return live; }
 long alloc_refused(void) { return refused; }
@@ -22,8 +22,8 @@ long alloc_refused(void) { return refused; }
 static int refuse(size_t n) {
   int r = 0;
   pthread_mutex_lock(&lock);
-  if (fail_next >= 0 && fail_next-- == 0) r = 1;
-  if (limit && live + n > limit) r = 1;
+  if (granted == 0 || (limit && live + n > limit)) r = 1;
+  if (granted > 0 && !r) --granted;
   refused += r;
   pthread_mutex_unlock(&lock);
   return r;

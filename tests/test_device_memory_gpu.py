@@ -3,17 +3,20 @@ tests/native/alloc_limit.c before the CUDA runtime, which refuses allocations.
 
 A call that cannot have its memory reports it, leaves the handle as it was and
 works once there is room; what a call allocates together it has whole or not at
-all.
+all.  The step's slot maps are optional: they are given back to whatever else needs
+the room, and the results are the same without them.
 """
 import ctypes as C
 import os
 import subprocess
 import sys
+import threading
 
 import numpy as np
 import pytest
 
 from cupf_b200 import abi, cases
+from cupf_b200.dense import DenseSolver
 from cupf_b200.solver import APTSolver
 
 pytestmark = pytest.mark.gpu
@@ -41,16 +44,19 @@ def child(built, tmp_path_factory):
 
 def shim():
     s = C.CDLL(None)
-    s.alloc_fail_next.argtypes = [C.c_long]
+    s.alloc_refuse_from.argtypes = [C.c_long]
     s.alloc_limit.argtypes = [C.c_size_t]
     s.alloc_live.restype = C.c_size_t
     s.alloc_refused.restype = C.c_long
     return s
 
 
-def refused(call, *args):
+def refused(a, n, call, *args):
+    """The call with all but its first n allocations refused."""
+    a.alloc_refuse_from(n)
     with pytest.raises(abi.CupfError) as e:
         call(*args)
+    a.alloc_refuse_from(-1)
     assert e.value.status == OOM
 
 
@@ -80,11 +86,9 @@ def scratch_refused():
         s.init_from_argmax(c.phi, c.alpha)
         s.step(30)
         for n in (0, 1):
-            a.alloc_fail_next(n)
-            refused(s.set_slots, ph, low, 0)
+            refused(a, n, s.set_slots, ph, low, 0)
             s.step(7)
-            a.alloc_fail_next(n)
-            refused(s.get_slots)
+            refused(a, n, s.get_slots)
         s.step(7)
         same(s.get_slots(), want)
         s.set_slots(ph, ids, 30)
@@ -94,18 +98,16 @@ def scratch_refused():
 
 def moves(solver, c, a):
     """Steps and frame moves, the second past the archive's first capacity; with `a`
-    every allocation on the way is refused once."""
+    every allocation on the way is refused at first."""
     solver.step(20)
     for n in (0, 1) if a else ():
-        a.alloc_fail_next(n)
-        refused(solver.move_domain, 1, 10 ** 6, 0)
+        refused(a, n, solver.move_domain, 1, 10 ** 6, 0)
     tip, _, _ = solver.move_domain(1, 10 ** 6, 0)
     out = [solver.move_domain(tip, tip - 2, 0)]
     solver.step(9)
     mc = 4 * c.params.fnz + 5  # two layers fit, four more are moved
     if a:
-        a.alloc_fail_next(0)
-        refused(solver.move_domain, tip, tip - 3, mc)
+        refused(a, 0, solver.move_domain, tip, tip - 3, mc)
     out.append(solver.move_domain(tip, tip - 3, mc))
     assert out[0][2] >= 3 and out[1][2] >= 4
     solver.step(9)
@@ -134,14 +136,12 @@ def volumes_and_nuclei_refused():
         s.step(5)
         _, alpha = s.collect(clear=True)
         for n in (0, 1):
-            a.alloc_fail_next(n)
-            refused(s.grain_volumes, p.num_theta)
+            refused(a, n, s.grain_volumes, p.num_theta)
         v = s.grain_volumes(p.num_theta)
         inner = alpha.reshape(p.fnz, p.fny, p.fnx)[1:-1, 1:-1, 1:-1]
         assert np.array_equal(v[1:], np.bincount(inner.ravel(), minlength=p.num_theta + 1)[1:])
         for n in (0, 1, 2):
-            a.alloc_fail_next(n)
-            refused(s.nucl_init)
+            refused(a, n, s.nucl_init)
         s.nucl_init()
         s.nucleate()
         s.step(2)
@@ -150,4 +150,96 @@ def volumes_and_nuclei_refused():
 
 @pytest.mark.parametrize("name", ["scratch_refused", "archive_refused", "volumes_and_nuclei_refused"])
 def test_refused_allocations_leave_the_handle_whole(child, name):
+    child(name)
+
+
+def map_bytes(p, precision="fp32"):
+    align = 2 if precision == "fp32" else 4
+    return -(-p.fnx // align) * align * p.fny * p.fnz * (4 * p.num_pf + 2)
+
+
+def whole_run(s, c, state):
+    """Every call that allocates on the way."""
+    s.set_slots(*state, 0)
+    s.step(20)
+    tip, mc, _ = s.move_domain(1, 10 ** 6, 0)
+    moved = s.move_domain(tip, tip - 1, mc)
+    s.step(11)
+    phi, alpha = s.collect(clear=True)
+    return (moved, alpha, phi, s.grain_volumes(c.params.num_theta), s.qoi_sums(),
+            *s.get_slots())
+
+
+def equal(a, b):
+    for u, v in zip(a, b):
+        assert np.array_equal(np.asarray(u), np.asarray(v))
+
+
+def maps_give_way():
+    """A device that holds the simulation and all it allocates later, but not its maps
+    too: every call succeeds, for this handle, a second one and the full-PF solver."""
+    a, c = shim(), line()
+    with APTSolver(c) as s:
+        s.init_from_argmax(c.phi, c.alpha)
+        state = s.get_slots()
+    for prec in ("fp32", "fp16"):
+        with APTSolver(c, precision=prec) as s:
+            want = whole_run(s, c, state)
+            need = a.alloc_live() - map_bytes(c.params, prec)
+        a.alloc_limit(need + 4096)
+        with APTSolver(c, precision=prec) as s:
+            held = a.alloc_live()
+            got = whole_run(s, c, state)
+            assert a.alloc_refused() > 0
+            assert a.alloc_live() == need
+        equal(got, want)
+        # the maps were there before the scratch was
+        with APTSolver(c, precision=prec) as s:
+            s.init_from_argmax(c.phi, c.alpha)
+            assert a.alloc_live() == held
+        # refused from the start: the same states
+        a.alloc_limit(held - 1)
+        with APTSolver(c, precision=prec) as s:
+            assert a.alloc_live() == held - map_bytes(c.params, prec)
+            a.alloc_limit(0)
+            equal(whole_run(s, c, state), want)
+    a.alloc_limit(2 * need + 4096)
+    with APTSolver(c, precision="fp16") as s, APTSolver(c, precision="fp16") as t:
+        equal(whole_run(s, c, state), want)
+        equal(whole_run(t, c, state), want)
+    a.alloc_limit(0)
+    d = cases.line_case(24, 24, 32, num_pf=1, num_grains=6, seed=1)
+    with DenseSolver(d):
+        full = a.alloc_live()
+    with APTSolver(c) as s:
+        s.init_from_argmax(c.phi, c.alpha)
+        a.alloc_limit(a.alloc_live() + full - 1)
+        with DenseSolver(d):
+            s.step(5)
+            s.sync()
+
+
+def maps_give_way_across_threads():
+    """A second simulation created while the first is stepping in another thread."""
+    a, c = shim(), line()
+    with APTSolver(c) as s:
+        s.init_from_argmax(c.phi, c.alpha)
+        s.step(1000)
+        want = s.collect(clear=True)
+        need = a.alloc_live() - map_bytes(c.params)
+    a.alloc_limit(2 * need + 4096)
+    with APTSolver(c) as s:
+        s.init_from_argmax(c.phi, c.alpha)
+        go = threading.Thread(target=lambda: [s.step(10) for _ in range(100)])
+        go.start()
+        with APTSolver(c) as t:
+            t.init_from_argmax(c.phi, c.alpha)
+            t.step(1000)
+            equal(t.collect(clear=True), want)
+        go.join()
+        equal(s.collect(clear=True), want)
+
+
+@pytest.mark.parametrize("name", ["maps_give_way", "maps_give_way_across_threads"])
+def test_slot_maps_give_way(child, name):
     child(name)
