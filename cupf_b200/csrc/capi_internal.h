@@ -24,6 +24,8 @@ cupf_status cupf_fail(cupf_status st, const char* fmt, ...);
 // optional memory: a simulation without them merges every cell every step, with the
 // same results.
 bool release_slot_maps();
+// Bytes that release_slot_maps could free on `device`.
+size_t held_slot_map_bytes(int device);
 
 // An allocation that the slot maps give way to: run again after each release while the
 // device is out of memory.  A failure is reported by the return value, not by the next

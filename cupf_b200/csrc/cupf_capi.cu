@@ -387,13 +387,25 @@ bool release_slot_maps() {
   return false;
 }
 
+static size_t map_bytes(const cupf_apt_handle* h) {
+  return (size_t)h->g.ss * (h->g.np * sizeof(uint32_t) + 2);
+}
+
+size_t held_slot_map_bytes(int device) {
+  std::lock_guard<std::mutex> lock(g_map_mutex);
+  size_t n = 0;
+  for (const cupf_apt_handle* h : g_map_owners)
+    if (h->device == device) n += map_bytes(h);
+  return n;
+}
+
 // Slot maps and change marks of the step (a quarter of the FP32 pair buffers' size).
 // A grid whose pairs leave no room for them runs without, and they are given back
 // when any other allocation of the library needs the room (release_slot_maps): every
 // cell is then merged every step, with the same results.
 static cupf_status alloc_maps(cupf_apt_handle* h) {
   const size_t cells = (size_t)h->g.ss;
-  const size_t bytes = cells * (h->g.np * sizeof(uint32_t) + 2);
+  const size_t bytes = map_bytes(h);
   size_t room = ~(size_t)0, total = 0;
   if (bytes > kMapReserve / 64) CK(cudaMemGetInfo(&room, &total));  // the query takes 80 us
   if (room - bytes < kMapReserve || room < bytes ||

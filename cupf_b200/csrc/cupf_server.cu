@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cstddef>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -89,7 +90,7 @@ struct Request {
   uint8_t* dquiet[2] = {nullptr, nullptr};  // quiet-item flags of each buffer
   uint32_t* dmap = nullptr;                 // slot maps (StepArgs::map), or NULL
   uint8_t* dredo[2] = {nullptr, nullptr};   // change marks of each buffer
-  size_t bytes = 0;
+  size_t bytes = 0, map_bytes = 0;  // device memory: required, and that of its slot maps
   int zc = 64, ty = 8, ntx = 0, nty = 0, nzc = 0;
   // results
   HostBuf hres;  // argmax grain ids, res_len values
@@ -108,7 +109,8 @@ struct cupf_server {
   std::deque<int64_t> queue;
   std::map<int64_t, std::unique_ptr<Request>> reqs;
   std::vector<int64_t> slots;  // request id per slot (0 = free)
-  size_t used_bytes = 0;
+  size_t used_bytes = 0;  // required memory of the resident requests
+  size_t map_bytes = 0;   // their slot maps' memory, which gives way to any request's required
   size_t budget = 0;
   BatchSim* d_sims = nullptr;
   CUtensorMap* d_tmaps = nullptr;
@@ -195,9 +197,48 @@ static void put_host(cupf_server* s, HostBuf* b) {
   *b = HostBuf();
 }
 
+// Take the slot maps of the resident request with the largest ones (false: none has
+// any): its cells are merged every step from here on, with the same results.  The
+// batched step reads the pointer from the device's BatchSim, so the captured graph
+// stays as it is.
+static bool drop_maps(cupf_server* s) {
+  Request* r = nullptr;
+  for (int64_t id : s->slots) {
+    Request* q = id ? s->reqs[id].get() : nullptr;
+    if (q && q->dmap && (!r || q->map_bytes > r->map_bytes)) r = q;
+  }
+  if (!r) return false;
+  cudaMemsetAsync(reinterpret_cast<char*>(s->d_sims + r->slot) + offsetof(BatchSim, a) +
+                      offsetof(StepArgs, map),
+                  0, sizeof(StepArgs::map), s->stream);
+  for (void* p : {(void*)r->dmap, (void*)r->dredo[0], (void*)r->dredo[1]}) cudaFreeAsync(p, s->stream);
+  r->dmap = nullptr;
+  r->dredo[0] = r->dredo[1] = nullptr;
+  s->map_bytes -= r->map_bytes;
+  r->map_bytes = 0;
+  return true;
+}
+
+// The same where the device is out of memory: what the pool holds free goes back too.
+static bool drop_maps_to_device(cupf_server* s) {
+  if (!drop_maps(s)) return false;
+  cudaStreamSynchronize(s->stream);
+  cudaMemPoolTrimTo(s->pool, 0);
+  return true;
+}
+
+// An allocation the server needs: every slot map gives way to it.
+template <class F>
+static cudaError_t with_room(cupf_server* s, F&& allocate) {
+  for (;;) {
+    const cudaError_t e = with_room(allocate);
+    if (e != cudaErrorMemoryAllocation || !drop_maps_to_device(s)) return e;
+  }
+}
+
 // A request's device buffer from the server's pool, ordered on its stream.
 static cudaError_t pool_alloc(cupf_server* s, void** p, size_t n) {
-  return cudaMallocFromPoolAsync(p, n, s->pool, s->stream);
+  return with_room(s, [&] { return cudaMallocFromPoolAsync(p, n, s->pool, s->stream); });
 }
 
 // Return a request's buffers to the pool (ordered after the work queued on the
@@ -227,8 +268,8 @@ static size_t request_bytes(const cupf_apt_params& p, int pair_bytes, int num_pf
 }
 
 // Bytes of a request's slot maps and change marks.  They are not part of
-// request_bytes: a request is admitted without them where the budget has no room
-// (its cells are then merged every step, with the same results).
+// request_bytes and never weigh in a request's admission: it gets them where the budget
+// has room, and loses them to a later request's required memory (drop_maps).
 static size_t map_bytes(const cupf_apt_params& p, int pair_bytes, int num_pf) {
   const int palign = pair_bytes == 8 ? 2 : 4;
   const size_t xp = (p.fnx + palign - 1) / palign * palign;
@@ -256,8 +297,11 @@ static std::pair<int, int> autotune_tile(cupf_server* s, const Request* r) {
     const int nz = r->p.fnz - 2;
     const int cand[] = {8, 16, 32, 64, 128, 256};
     cupf_apt_handle* h = nullptr;
-    if (cupf_apt_create(&r->p, &in, s->cfg.device, (cupf_precision)s->cfg.precision, &h) ==
-        CUPF_OK) {
+    cupf_status made;
+    do {
+      made = cupf_apt_create(&r->p, &in, s->cfg.device, (cupf_precision)s->cfg.precision, &h);
+    } while (made == CUPF_ERR_OOM && drop_maps_to_device(s));
+    if (made == CUPF_OK) {
       for (int ty : {8, 4}) {
         if (fixed_ty && ty != fixed_ty) continue;
         if (cupf_apt_set_tile(h, ty) != CUPF_OK) continue;
@@ -341,20 +385,32 @@ static cupf_status admit(cupf_server* s, Request* r, int slot) {
     CK(cudaMemsetAsync(r->dquiet[b], 0, nq, st));
   }
   r->bytes = request_bytes(p, s->pair_bytes, np);
-  // slot maps where the budget holds them beside this and every queued request
+  // slot maps where the budget holds them beside this and every queued request, and
+  // the device has the room
   {
     const size_t extra = map_bytes(p, s->pair_bytes, np);
-    size_t want = s->used_bytes + r->bytes + extra;
+    size_t want = s->used_bytes + s->map_bytes + r->bytes + extra;
     for (int64_t q : s->queue) want += request_bytes(s->reqs[q]->p, s->pair_bytes, np);
-    if (want <= s->budget) {
-      const size_t cells = (size_t)r->g.ss;
-      CK(pool_alloc(s, (void**)&r->dmap, cells * np * sizeof(uint32_t)));
+    const size_t cells = (size_t)r->g.ss;
+    const size_t part[3] = {cells * np * sizeof(uint32_t), cells, cells};
+    void* m[3] = {nullptr, nullptr, nullptr};
+    cudaError_t got = want <= s->budget ? cudaSuccess : cudaErrorMemoryAllocation;
+    for (int b = 0; b < 3 && got == cudaSuccess; ++b) {
+      got = cudaMallocFromPoolAsync(&m[b], part[b], s->pool, st);
+      if (got != cudaSuccess) m[b] = nullptr;
+    }
+    if (got == cudaSuccess) {
+      r->dmap = static_cast<uint32_t*>(m[0]);
       CK(cudaMemsetAsync(r->dmap, 0xFF, cells * sizeof(uint32_t), st));  // nothing known
       for (int b = 0; b < 2; ++b) {
-        CK(pool_alloc(s, (void**)&r->dredo[b], cells));
+        r->dredo[b] = static_cast<uint8_t*>(m[1 + b]);
         CK(cudaMemsetAsync(r->dredo[b], 0, cells, st));
       }
-      r->bytes += extra;
+      r->map_bytes = extra;
+    } else {
+      for (void* p_ : m)
+        if (p_) cudaFreeAsync(p_, st);
+      cudaGetLastError();
     }
   }
   // initial state in both buffers
@@ -467,6 +523,7 @@ static cupf_status admit(cupf_server* s, Request* r, int slot) {
   r->t_admit = now_s();
   s->slots[slot] = r->id;
   s->used_bytes += r->bytes;
+  s->map_bytes += r->map_bytes;
   s->dirty = true;
   return CUPF_OK;
 }
@@ -482,8 +539,10 @@ static cupf_status retire(cupf_server* s, Request* r, int cur) {
     if (s->d_counts) cudaFree(s->d_counts);
     if (s->d_first) cudaFree(s->d_first);
     s->counts_cap = 0;
-    CK(malloc_together({{(void**)&s->d_counts, (ng + 1) * sizeof(unsigned long long)},
-                        {(void**)&s->d_first, (ng + 1) * sizeof(long long)}}));
+    CK(with_room(s, [&] {
+      return malloc_together({{(void**)&s->d_counts, (ng + 1) * sizeof(unsigned long long)},
+                              {(void**)&s->d_first, (ng + 1) * sizeof(long long)}});
+    }));
     s->counts_cap = ng + 1;
   }
   CK(cudaMemsetAsync(s->d_counts, 0, (ng + 1) * sizeof(unsigned long long), st));
@@ -527,6 +586,8 @@ static cupf_status retire(cupf_server* s, Request* r, int cur) {
   r->res_qoi[2] = v / ((double)(g.fnx - 2) * (g.fny - 2));
   free_request_device(s, r);
   s->used_bytes -= r->bytes;
+  s->map_bytes -= r->map_bytes;
+  r->map_bytes = 0;
   s->slots[r->slot] = 0;
   r->slot = -1;
   r->state = DONE;
@@ -566,7 +627,7 @@ static cupf_status rebuild(cupf_server* s) {
     if (s->d_items) cudaFree(s->d_items);
     const int cap = std::max(s->nitems, 2 * s->items_cap);
     s->items_cap = 0;
-    CK(malloc_together({{(void**)&s->d_items, cap * sizeof(int4)}}));
+    CK(with_room(s, [&] { return malloc_together({{(void**)&s->d_items, cap * sizeof(int4)}}); }));
     s->items_cap = cap;
   }
   if (s->nitems)
@@ -677,6 +738,7 @@ extern "C" cupf_status cupf_server_create(const cupf_server_config* cfg, cupf_se
   size_t fr = 0, tot = 0;
   CK(cudaMemGetInfo(&fr, &tot));
   const size_t reserve = (size_t)2 << 30;
+  fr += held_slot_map_bytes(cfg->device);  // they give way to requests
   const size_t avail = fr > reserve ? fr - reserve : 0;
   s->budget = cfg->hbm_budget_bytes > 0 ? std::min((size_t)cfg->hbm_budget_bytes, avail) : avail;
   *out = s.release();
@@ -792,6 +854,8 @@ extern "C" cupf_status cupf_server_pump(cupf_server* s, int32_t* n_running, int3
       }
     const size_t need = request_bytes(r->p, s->pair_bytes, s->cfg.num_pf);
     if (slot < 0 || s->used_bytes + need > s->budget) break;
+    while (s->used_bytes + s->map_bytes + need > s->budget && drop_maps(s)) {
+    }
     s->queue.pop_front();
     if ((e = admit(s, r, slot))) {
       free_request_device(s, r);

@@ -17,6 +17,7 @@ import pytest
 
 from cupf_b200 import abi, cases
 from cupf_b200.dense import DenseSolver
+from cupf_b200.server import Server
 from cupf_b200.solver import APTSolver
 
 pytestmark = pytest.mark.gpu
@@ -242,4 +243,98 @@ def maps_give_way_across_threads():
 
 @pytest.mark.parametrize("name", ["maps_give_way", "maps_give_way_across_threads"])
 def test_slot_maps_give_way(child, name):
+    child(name)
+
+
+RUNNING = 1
+REQUESTS = [((48, 44, 40), 1), ((40, 56, 48), 2), ((56, 40, 64), 3)]
+
+
+def request(shape, seed):
+    return cases.line_case(*shape, num_pf=8, num_grains=20, seed=seed)
+
+
+def required(c, precision):
+    """Bytes a request is admitted by (its maps are not among them)."""
+    p = c.params
+    pair, align = (8, 2) if precision == "fp32" else (4, 4)
+    xp = -(-p.fnx // align) * align
+    return (2 * xp * p.fny * p.fnz * p.num_pf * pair + p.fnx * p.fny * p.fnz * 8 +
+            2 * -(-(p.fnx - 2) // 32) * -(-(p.fny - 2) // 4) * (p.fnz - 2) + 4096)
+
+
+def server(precision, **kw):
+    return Server(precision=precision, steps_per_round=16, autotune=False, **kw)
+
+
+def alone(cs, precision):
+    out = []
+    for c in cs:
+        with server(precision) as srv:
+            r = srv.submit(c, 70)
+            srv.run_until_done([r])
+            out.append(srv.result(r))
+    return out
+
+
+def check_results(srv, rids, want):
+    srv.run_until_done(rids)
+    for r, w in zip(rids, want):
+        got = srv.result(r)
+        assert np.array_equal(got["alpha"], w["alpha"]) and got["qoi"] == w["qoi"]
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+def test_maps_never_hold_up_a_later_request(built, precision):
+    """Requests that fit the budget together, submitted one after the other while the
+    earlier ones hold slot maps, are all resident at once."""
+    cs = [request(*r) for r in REQUESTS]
+    want = alone(cs, precision)
+    need = [required(c, precision) for c in cs]
+    assert need[0] + map_bytes(cs[0].params, precision) <= sum(need[:2])
+    for several in (2, 3):
+        with server(precision, hbm_budget_bytes=sum(need[:several])) as srv:
+            rids = []
+            for c in cs[:several]:
+                rids.append(srv.submit(c, 70))
+                srv.pump()
+                assert srv.status(rids[-1]) == RUNNING
+            check_results(srv, rids, want)
+
+
+def served_without_map_memory():
+    """The device refuses the maps' memory to a request, or needs a resident one's back
+    for the next: both requests run, with the same results."""
+    a = shim()
+    cs = [request(*r) for r in REQUESTS[:2]]
+    for precision in ("fp32", "fp16"):
+        want = alone(cs, precision)
+        maps = [map_bytes(c.params, precision) for c in cs]
+        with server(precision) as srv:
+            empty = a.alloc_live()
+            rids = []
+            held = []
+            for c in cs:
+                rids.append(srv.submit(c, 70))
+                srv.pump()
+                held.append(a.alloc_live())
+            check_results(srv, rids, want)
+        for limit in (held[0] - 1, held[0] - maps[0] // 2, held[1] - sum(maps) + 65536):
+            before = a.alloc_refused()
+            with server(precision) as srv:
+                assert a.alloc_live() <= empty
+                rids = [srv.submit(cs[0], 70)]
+                a.alloc_limit(limit)
+                srv.pump()
+                a.alloc_limit(held[1] - sum(maps) + 65536)
+                rids.append(srv.submit(cs[1], 70))
+                srv.pump()
+                assert [srv.status(r) for r in rids] == [RUNNING, RUNNING]
+                assert a.alloc_refused() > before
+                a.alloc_limit(0)
+                check_results(srv, rids, want)
+
+
+@pytest.mark.parametrize("name", ["served_without_map_memory"])
+def test_server_without_map_memory(child, name):
     child(name)
