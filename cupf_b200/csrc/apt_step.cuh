@@ -31,14 +31,17 @@
 // beside the pairs: a step merges again only the cells whose own or face
 // neighbours' lists changed in the step before.  Whoever changes a cell's list
 // marks the cells that read it (mark_readers) for the next step; whoever replaces
-// the whole state invalidates every map.  Merges are done by the warp together,
-// four cells a pass with a lane per stencil point, so a few scattered cells do not
-// hold up a warp's other lanes.
+// the whole state invalidates every map.  A few marked cells are merged by the warp
+// together, four a pass with a lane per stencil point, so that scattered cells do not
+// hold up a warp's other lanes; a row that is nearly all marked by its own lanes
+// (kRowMerge), as every row is where the device has no room for maps.
 //
-// What bounds it: instruction issue and latency, not bytes.  On 128x128x256, NUM_PF = 8
-// (B200, us per step over steps 51-150, all-empty items left alone): FP32 227 with
-// a merge of every cell, 151 with the maps; FP16 196 and 138.  In the first 50 steps, when
-// a quarter of the cells and more are merged, FP32 219 and 195, FP16 187 and 171.
+// What bounds it: instruction issue and latency, not bytes.  128x128x256 line case, NUM_PF
+// = 8, on a B200, us per step over steps 1-20, 21-50 and 51-150 (all-empty items left
+// alone): FP32 220, 181, 163, where no maps are kept 273, 286, 286, and with the merge of
+// every cell that the maps replaced 213, 232, 230; FP16 202, 156, 144; 231, 236, 242; 182,
+// 200, 198.  In the first steps, while every grain's tail grows a cell a step, a quarter
+// of the cells and more are merged: there the maps cost more than they save.
 //
 // The reference's aliasing write on merge overflow (local_phs[s][NUM_PF] ==
 // local_phs[s+1][0]) is restated: such cells are merged every step.
@@ -221,6 +224,106 @@ struct CtaSmem {
   }
 };
 
+// The merge of one cell by its own lane: the first-seen order over (D,B,L,C,R,T,U) x
+// slot.  Writes the cell's slot-map words to wcol and returns what the warp's merge
+// (step_item) does: the slot count in bits 28..31, merge overflows aliased (low byte)
+// and dropped (second byte), a list of the centre's that loses a grain (bit 16), an
+// overflow (bit 17), with its alias word second.  pD, pC, pU: the cell in its planes.
+//
+// The list starts as the point below's.  An entry of another point whose grain stands
+// in that same slot needs no search (a cell's slots stand in the first-seen order of
+// its own neighbourhood, which starts with the column); the few others are looked up
+// one by one, in order.
+template <int NP, class S, int BW, int BCELLS>
+__device__ __forceinline__ uint2 merge_cell(const typename S::T* pD, const typename S::T* pC,
+                                            const typename S::T* pU, uint32_t* wcol) {
+  auto point = [&](int s) {
+    return s == 0 ? pD : s == 6 ? pU : pC + (s == 1 ? -BW : s == 2 ? -1 : s == 4 ? 1 : s == 5 ? BW : 0);
+  };
+  int list[NP];  // the grains placed so far; below -1: none
+  uint32_t occ = 0;
+  bool odd = false;  // a hole or a repeated grain in the list of the point below
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    const int id = S::id(pD[p * BCELLS]);
+    occ |= (uint32_t)(id != -1) << p;
+    list[p] = id != -1 ? id : -2 - p;
+#pragma unroll
+    for (int q = 0; q < p; ++q) odd = odd || list[p] == list[q];
+  }
+  odd = odd || (occ & (occ + 1)) != 0;
+  uint32_t todo[2] = {odd ? occ : 0u, 0u};  // entries to look up: 8 bits a point, 4 points a word
+  int cnt = odd ? 0 : __popc(occ);
+  uint32_t w[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    if (odd) list[p] = -2;
+    w[p] = (uint32_t)NP * 0x1111111u;
+    if (list[p] >= 0) w[p] -= (uint32_t)(NP - p);
+  }
+#pragma unroll
+  for (int s = 1; s < 7; ++s) {
+    const typename S::T* pt = point(s);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int id = S::id(pt[p * BCELLS]);
+      if (id == list[p]) w[p] -= (uint32_t)(NP - p) << (4 * s);
+      if (id != list[p] && id != -1) todo[s >> 2] |= 1u << (8 * (s & 3) + p);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < NP; ++p) wcol[p * 32] = w[p];
+  uint32_t info = 0, al = 0xFFFFFFFFu;
+  while (todo[0] | todo[1]) {
+    const bool hi = todo[0] == 0;
+    const int b = __ffs(hi ? todo[1] : todo[0]) - 1;
+    if (hi)
+      todo[1] &= todo[1] - 1;
+    else
+      todo[0] &= todo[0] - 1;
+    const int s = (b >> 3) + (hi ? 4 : 0), p = b & 7;
+    const int id = S::id(point(s)[p * BCELLS]);
+    int j = cnt;
+#pragma unroll
+    for (int q = NP - 1; q >= 0; --q)
+      if (list[q] == id) j = q;
+    if (j == NP) {  // overflow: the last entry's value is the one aliased
+      info = (info | 1u << 17 | (uint32_t)(s == 3) << 16) + (s < 6 ? 1u : 0x100u);
+      if (s < 6) al = (al & ~(0xFu << (4 * s + 4))) | ((uint32_t)p << (4 * s + 4));
+      continue;
+    }
+    if (j == cnt) {
+#pragma unroll
+      for (int q = 0; q < NP; ++q)
+        if (q == j) list[q] = id;
+      ++cnt;
+    }
+    // the last slot holding the id, as the reference's later write wins; an id repeated
+    // in the centre's list does not survive the step
+    const uint32_t old = wcol[j * 32], at = map_code(old, s);
+    if (at == (uint32_t)NP) {
+      wcol[j * 32] = old - ((uint32_t)(NP - p) << (4 * s));
+    } else {
+      if ((uint32_t)p > at) wcol[j * 32] = old + (((uint32_t)p - at) << (4 * s));
+      info |= (uint32_t)(s == 3) << 16;
+    }
+  }
+  if (info & (1u << 17)) {
+    // a point's own grain of slot 0 overwrites the value aliased there
+#pragma unroll
+    for (int s = 1; s < 7; ++s)
+      if (map_code(wcol[0], s) != (uint32_t)NP) al |= 0xFu << (4 * s);
+  }
+  return make_uint2(info | ((uint32_t)cnt << 28), al);
+}
+
+// The same out of line, where it runs seldom.
+template <int NP, class S, int BW, int BCELLS>
+__device__ __noinline__ uint2 merge_cell_call(const typename S::T* pD, const typename S::T* pC,
+                                              const typename S::T* pU, uint32_t* wcol) {
+  return merge_cell<NP, S, BW, BCELLS>(pD, pC, pU, wcol);
+}
+
 // One work item: the column tile (txi, tyi) over the z chunk zci of one
 // simulation.  qbase is the CTA's running plane sequence number: plane q of
 // this item is sequence number qbase + q, which fixes its stage (mod STAGES)
@@ -236,6 +339,16 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
   constexpr int BW = Smem::BW;
   constexpr int BCELLS = Smem::BCELLS;
   constexpr bool kDec = Smem::kDecode;
+  // A row with more marked cells than this is merged by its own lanes, at about the cost
+  // of seven passes of four cells (0: only where no maps are kept).  Measured on a B200, us
+  // per step over the first 20 steps and over steps 51-150, NUM_PF = 8: FP32 28: line
+  // 128x128x256 220 and 163, pool 256x256x768 5200 and 4620; 24: 222, 163, 5216, 4632; with
+  // passes only 233, 164, 5380, 4673.  In 16-bit pairs, whose pool's FP64 model leaves little
+  // of the instruction cache, 28: 198, 144, 5241, 4597, with passes only 202, 144, 5114, 4414;
+  // there it is a call, too: inline it costs the pool 4963 where it is never taken.
+  // Without maps: FP32 line 317 with passes only, 286 by lanes, pool 7611 and 5894; FP16
+  // 276 and 242, 7000 and 5667.
+  constexpr int kRowMerge = S::kBytes == 8 ? 28 : 0;
   constexpr unsigned FULL = 0xffffffffu;
   // offsets of the centre plane's stencil points B, L, C, R, T from the cell
   constexpr int ctr_off[7] = {0, -BW, -1, 0, 1, BW, 0};
@@ -392,13 +505,24 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
     const P* plU = stages + (size_t)sU * Smem::kStagePairs;
 
     // ---- merge of the warp's marked cells: first-seen order over (D,B,L,C,R,T,U) x
-    // slot.  Eight lanes take a cell, lane s the list of point s; each turn places
-    // the first grain not placed yet, and every lane finds the slot it has in its
+    // slot.  In a pass eight lanes take a cell, lane s the list of point s; each turn
+    // places the first grain not placed yet, and every lane finds the slot it has in its
     // own list.  The turns give a word per point; its transpose the words per slot.
     uint32_t alias = 0xFFFFFFFFu;  // slot at point s-1 whose value sits in slot 0 of point s
     bool force_mark = false;
     uint32_t todo = __ballot_sync(FULL, need);
-    if (todo) {
+    uint32_t info = 0;
+    if (todo && (!a.map || (kRowMerge && __popc(todo) > kRowMerge))) {
+      if (need) {  // most of the row, or every cell of every step: a lane per cell
+        uint2 r;
+        if constexpr (kRowMerge != 0)
+          r = merge_cell<NP, S, BW, BCELLS>(plD + c, stC + c, plU + c, wcol);
+        else
+          r = merge_cell_call<NP, S, BW, BCELLS>(plD + c, stC + c, plU + c, wcol);
+        info = r.x;
+        if (info & (1u << 17)) alias = r.y;
+      }
+    } else if (todo) {
       const P* mp = (m_pt == 0 ? plD : m_pt == 6 ? plU : stC) + m_off;
       do {
         int src = -1;  // the pass's cells: the lowest four marked lanes
@@ -438,7 +562,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
           cnt += mine != 0;
         }
         // an id repeated in the centre's list does not survive the step
-        uint32_t info = (uint32_t)cnt << 28;
+        uint32_t res = (uint32_t)cnt << 28;
         if (__any_sync(FULL, un | (m_pt == 3 ? dup : 0u))) {
           // merge overflow: local_phs[s][NUM_PF] aliases local_phs[s+1][0], which
           // point s+1's own grain of slot 0 overwrites; past the array at s == 6
@@ -456,7 +580,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
             q += __shfl_xor_sync(FULL, q, d);
             f |= __shfl_xor_sync(FULL, f, d);
           }
-          info |= q | f;
+          res |= q | f;
           if (src >= 0 && m_pt == 7) wbuf[(NP + 1) * 32 + src] = al;
         }
         // transpose the eight lanes' 4-bit fields: lane j gets slot j's word
@@ -469,31 +593,30 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
         }
         if (src >= 0) {
           if (m_pt < NP) wbuf[m_pt * 32 + src] = codes;
-          if (m_pt == 7) wbuf[NP * 32 + src] = info;
+          if (m_pt == 7) wbuf[NP * 32 + src] = res;
         }
       } while (todo);
       __syncwarp();
       if (need) {
-        const uint32_t info = wbuf[NP * 32 + lane];
-        n = (int)(info >> 28);
-        uint32_t mark0 = (uint32_t)n;
-        if (info & 0x3FFFFu) {
-          force_mark = (info >> 16) & 1u;
-          n_ovf += (info & 0xFFu) + ((info & 0xFF00u) << 8);
-          if (info & (1u << 17)) {
-            alias = wbuf[(NP + 1) * 32 + lane];
-            mark0 = kMapEveryStep;
-          }
-        }
-        if (a.map) {
-          a.map[cell] = (n ? wcol[0] : 0u) | (mark0 << 28);
-#pragma unroll
-          for (int j = 1; j < NP; ++j)
-            if (j < n) a.map[j * ss + cell] = wcol[j * 32];
-          if (had_mark) a.redo_in[cell] = 0;
-        }
+        info = wbuf[NP * 32 + lane];
+        if (info & (1u << 17)) alias = wbuf[(NP + 1) * 32 + lane];
       }
       __syncwarp();  // the buffer is rewritten at the next plane
+    }
+    if (need) {
+      n = (int)(info >> 28);
+      if (info & 0x3FFFFu) {
+        force_mark = (info >> 16) & 1u;
+        n_ovf += (info & 0xFFu) + ((info & 0xFF00u) << 8);
+      }
+      if (a.map) {
+        const uint32_t mark0 = info & (1u << 17) ? kMapEveryStep : (uint32_t)n;
+        a.map[cell] = (n ? wcol[0] : 0u) | (mark0 << 28);
+#pragma unroll
+        for (int j = 1; j < NP; ++j)
+          if (j < n) a.map[j * ss + cell] = wcol[j * 32];
+        if (had_mark) a.redo_in[cell] = 0;
+      }
     }
     copy_wait();
     if (!valid) continue;
@@ -510,12 +633,10 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
         if (hdy1) o[hdy1] = v;
       }
     };
-    if (n == 0) {
-      const P empty = S::empty();
 #pragma unroll
-      for (int p = 0; p < NP; ++p) put(p, empty);
-      continue;
-    }
+    for (int j = 0; j < NP; ++j)
+      if (j >= n) put(j, S::empty());
+    if (n == 0) continue;
 
     const P* pC = stC + c;
     const P* pts[7] = {plD + c, pC - BW, pC - 1, pC, pC + 1, pC + BW, plU + c};
@@ -633,10 +754,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
       return S::make(nv, oid);
     };
     // one loop body run to the cell's slot count (unrolled over NUM_PF it overruns the
-    // instruction cache: 165 against 142 us per step, FP32, 128x128x256, NUM_PF = 8)
-#pragma unroll
-    for (int j = 0; j < NP; ++j)
-      if (j >= n) put(j, S::empty());
+    // instruction cache: 1.16 times the time per step, FP32, 128x128x256, NUM_PF = 8)
     if (upd) {
 #pragma unroll 1
       for (int j = 0; j < n; ++j) {

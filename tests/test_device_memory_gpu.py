@@ -19,6 +19,7 @@ from cupf_b200 import abi, cases
 from cupf_b200.dense import DenseSolver
 from cupf_b200.server import Server
 from cupf_b200.solver import APTSolver
+from tests.test_slot_maps_gpu import SHAPES, crowded
 
 pytestmark = pytest.mark.gpu
 
@@ -241,7 +242,34 @@ def maps_give_way_across_threads():
         equal(s.collect(clear=True), want)
 
 
-@pytest.mark.parametrize("name", ["maps_give_way", "maps_give_way_across_threads"])
+def forms_of_the_merge():
+    """Crowded lists (holes, repeated ids, more grains than slots) with and without maps:
+    rows merged by the warp's passes, by their own lanes, and both."""
+    a = shim()
+    for interior, npf, bc in SHAPES:
+        c = cases.line_case(*interior, num_pf=npf, num_grains=12, seed=3, bc=bc)
+        ph, ids = crowded(c, npf, 12)
+        for prec in ("fp32", "fp16", "bf16"):
+            for tile in (8, 4):
+                got = []
+                for maps in (True, False):
+                    with APTSolver(c, precision=prec) as s:
+                        live = a.alloc_live()
+                    a.alloc_limit(0 if maps else live - 1)
+                    with APTSolver(c, precision=prec) as s:
+                        assert (a.alloc_live() == live) == maps
+                        a.alloc_limit(0)
+                        s.set_tile(tile)
+                        s.set_slots(ph, ids, 0)
+                        s.merge_overflows()
+                        s.step(11)
+                        got.append((s.merge_overflows(), *s.get_slots()))
+                    if not maps:
+                        equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("name", ["maps_give_way", "maps_give_way_across_threads",
+                                  "forms_of_the_merge"])
 def test_slot_maps_give_way(child, name):
     child(name)
 
