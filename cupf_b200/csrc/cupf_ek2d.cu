@@ -134,7 +134,7 @@ cupf_status launch_step(cupf_ek2d_handle* h, int prestep, uint32_t step) {
   return with_ek_storage(h->prec, [&](auto tag) -> cupf_status {
     using S = decltype(tag);
     if constexpr (sizeof(typename S::T) == 8)
-      CK(launch_dependent(h->stream, grid, MWARPS * 32, 0, ek2d_march_kernel<S>, a));
+      CK(launch_dependent(h->stream, grid, MWARPS * 32, 0, ek2d_march_kernel, a));
     else if (prestep)
       CK(launch_dependent(h->stream, grid, MWARPS * 32, 0, ek2d_march32_kernel<S, false>, a));
     else

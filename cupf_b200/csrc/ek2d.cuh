@@ -228,32 +228,31 @@ inline FluxConsts flux_consts(const EkArgs& a) {
   return c;
 }
 
-template <class T>
+// Constants of the FP64 step.
 struct Consts {
-  T k, omk, opk, hi, hiDl_half, eps, sqrt2, inv_sqrt2, lamd, dt, cosa, sina, a_s, epsilon, a_12, U0,
-      noise_amp;
+  double k, omk, opk, hi, hiDl_half, eps, sqrt2, inv_sqrt2, lamd, dt, cosa, sina, a_s, epsilon,
+      a_12, U0, noise_amp;
 };
 
-template <class T>
-__device__ __forceinline__ Consts<T> consts(const EkArgs& a) {
-  Consts<T> c;
-  c.k = (T)a.k;
-  c.omk = (T)1 - (T)a.k;
-  c.opk = (T)1 + (T)a.k;
-  c.hi = (T)a.hi;
-  c.hiDl_half = (T)a.hi * (T)a.Dl_tilde * (T)0.5;
-  c.eps = (T)a.eps;
-  c.sqrt2 = (T)a.sqrt2;
-  c.inv_sqrt2 = (T)1 / (T)a.sqrt2;
-  c.lamd = (T)a.lamd;
-  c.dt = (T)a.dt;
-  c.cosa = (T)a.cosa;
-  c.sina = (T)a.sina;
-  c.a_s = (T)a.a_s;
-  c.epsilon = (T)a.epsilon;
-  c.a_12 = (T)a.a_12;
-  c.U0 = (T)a.U0;
-  c.noise_amp = (T)a.noise_amp;
+__device__ __forceinline__ Consts consts(const EkArgs& a) {
+  Consts c;
+  c.k = a.k;
+  c.omk = 1.0 - (double)a.k;
+  c.opk = 1.0 + (double)a.k;
+  c.hi = a.hi;
+  c.hiDl_half = (double)a.hi * (double)a.Dl_tilde * 0.5;
+  c.eps = a.eps;
+  c.sqrt2 = a.sqrt2;
+  c.inv_sqrt2 = 1.0 / (double)a.sqrt2;
+  c.lamd = a.lamd;
+  c.dt = a.dt;
+  c.cosa = a.cosa;
+  c.sina = a.sina;
+  c.a_s = a.a_s;
+  c.epsilon = a.epsilon;
+  c.a_12 = a.a_12;
+  c.U0 = a.U0;
+  c.noise_amp = a.noise_amp;
   return c;
 }
 
@@ -271,8 +270,6 @@ template <>
 __device__ __forceinline__ double tanh_t<double>(double x) {
   return tanh(x);
 }
-__device__ __forceinline__ double div_t(double a, double b) { return a / b; }
-__device__ __forceinline__ double rsqrt_t(double x) { return 1.0 / sqrt(x); }
 
 // |phi| strictly inside the interface band, as the reference's
 // (double)phi > -0.995 && (double)phi < 0.995 (PF.cu:592): for a float, that
@@ -282,30 +279,28 @@ __device__ __forceinline__ bool in_band(double ph) { return fabs(ph) < 0.995; }
 
 // Anisotropy of the interface normal (phx, phz) rotated by the misorientation:
 // A = atheta (PF.cu:119-131), Ap = aptheta (PF.cu:135-146).
-template <class T>
-__device__ __forceinline__ void aniso(T phx, T phz, const Consts<T>& c, T& A, T& Ap) {
-  const T ux = c.cosa * phx + c.sina * phz;
-  const T uz = c.cosa * phz - c.sina * phx;
-  const T ux2 = ux * ux, uz2 = uz * uz;
-  const T m = ux2 + uz2;
+__device__ __forceinline__ void aniso(double phx, double phz, const Consts& c, double& A, double& Ap) {
+  const double ux = c.cosa * phx + c.sina * phz;
+  const double uz = c.cosa * phz - c.sina * phx;
+  const double ux2 = ux * ux, uz2 = uz * uz;
+  const double m = ux2 + uz2;
   if (m > c.eps) {
-    const T inv = div_t((T)1, m * m);
-    A = c.a_s * ((T)1 + c.epsilon * (ux2 * ux2 + uz2 * uz2) * inv);
+    const double inv = 1.0 / (m * m);
+    A = c.a_s * (1.0 + c.epsilon * (ux2 * ux2 + uz2 * uz2) * inv);
     Ap = -c.a_12 * ux * uz * (ux2 - uz2) * inv;
   } else {
-    A = (T)1;
-    Ap = (T)0;
+    A = 1.0;
+    Ap = 0.0;
   }
 }
 
-template <class T>
-__device__ __forceinline__ T aniso_a(T phx, T phz, const Consts<T>& c) {
-  const T ux = c.cosa * phx + c.sina * phz;
-  const T uz = c.cosa * phz - c.sina * phx;
-  const T ux2 = ux * ux, uz2 = uz * uz;
-  const T m = ux2 + uz2;
-  if (m > c.eps) return c.a_s * ((T)1 + c.epsilon * div_t(ux2 * ux2 + uz2 * uz2, m * m));
-  return (T)1;
+__device__ __forceinline__ double aniso_a(double phx, double phz, const Consts& c) {
+  const double ux = c.cosa * phx + c.sina * phz;
+  const double uz = c.cosa * phz - c.sina * phx;
+  const double ux2 = ux * ux, uz2 = uz * uz;
+  const double m = ux2 + uz2;
+  if (m > c.eps) return c.a_s * (1.0 + c.epsilon * ((ux2 * ux2 + uz2 * uz2) / (m * m)));
+  return 1.0;
 }
 
 // Write one cell's three values at (j, i) and at every halo cell that copies it:
@@ -342,23 +337,22 @@ __device__ __forceinline__ void put_with_halo(V* ps, V* U, V* D, int pitch, int 
 // J = A (A dpsi_n -+ Ap dpsi_t), the anisotropic psi flux of merge_PF
 // (PF.cu:475-538), and Uf, the solute flux with its anti-trapping part
 // (PF.cu:460-551).  kY selects the y-edge form (normal = z).
-template <bool kY, class T>
-__device__ __forceinline__ void edge_flux(const Consts<T>& c, bool merge, T psx, T psz, T phx,
-                                          T phz, T pha, T phb, T Ua, T Ub, T ja, T jb, T& J,
-                                          T& Uf) {
-  T A, Ap;
+template <bool kY>
+__device__ __forceinline__ void edge_flux(const Consts& c, bool merge, double psx, double psz,
+                                          double phx, double phz, double pha, double phb, double Ua,
+                                          double Ub, double ja, double jb, double& J, double& Uf) {
+  double A, Ap;
   aniso(phx, phz, c, A, Ap);
   J = kY ? A * (A * psz + Ap * psx) : A * (A * psx - Ap * psz);
   if (merge) {
-    const T n2 = phx * phx + phz * phz;
-    const T nn = (n2 > c.eps) ? (kY ? phz : phx) * rsqrt_t(n2) : (T)0;
-    Uf = c.hiDl_half * ((T)2 - pha - phb) * (Ub - Ua) + (T)0.5 * (ja + jb) * nn;
+    const double n2 = phx * phx + phz * phz;
+    const double nn = (n2 > c.eps) ? (kY ? phz : phx) * (1.0 / sqrt(n2)) : 0.0;
+    Uf = c.hiDl_half * (2.0 - pha - phb) * (Ub - Ua) + 0.5 * (ja + jb) * nn;
   }
 }
 
-template <class T>
-__device__ __forceinline__ T jat_of(const Consts<T>& c, T U, T ph, T D) {
-  return (T)0.5 * ((T)1 + c.omk * U) * ((T)1 - ph * ph) * D;
+__device__ __forceinline__ double jat_of(const Consts& c, double U, double ph, double D) {
+  return 0.5 * (1.0 + c.omk * U) * (1.0 - ph * ph) * D;
 }
 
 // Stored values of one cell's new psi, U and dpsi.
@@ -387,41 +381,39 @@ __device__ __forceinline__ void encode_cell(const EkArgs& a, bool merge, uint32_
 // One cell's update and stores (PF.cu:553-598): U' from the divergence of the
 // solute fluxes, then psi' with the new U, dpsi = rhs/tau_psi, the optional
 // noise term, and the stores with their halo copies.
-template <class S, class T = typename S::T, class V = typename S::V>
-__device__ __forceinline__ void cell_update(const EkArgs& a, const Consts<T>& c, bool merge,
-                                            uint32_t step_key, int gi, int gj, T psC, T phC, T UC,
-                                            T jatC, T JR, T JL, T JT, T JB, T UR, T UL, T UT, T UB,
-                                            T phR, T phL, T phT, T phB, T psR, T psL, T psT,
-                                            T psB, V* o_ps, V* o_U, V* o_D) {
-  T Un = UC;
+__device__ __forceinline__ void cell_update(const EkArgs& a, const Consts& c, bool merge, int gi,
+                                            int gj, double psC, double phC, double UC, double jatC,
+                                            double JR, double JL, double JT, double JB, double UR,
+                                            double UL, double UT, double UB, double phR, double phL,
+                                            double phT, double phB, double psR, double psL, double psT,
+                                            double psB, double* o_ps, double* o_U, double* o_D) {
+  double Un = UC;
   if (merge) {
-    const T rhsU = ((UR - UL) + (UT - UB)) * c.hi + c.sqrt2 * jatC;
-    const T tauU = c.opk - c.omk * phC;
-    Un = UC + c.dt * div_t(rhsU, tauU);
+    const double rhsU = ((UR - UL) + (UT - UB)) * c.hi + c.sqrt2 * jatC;
+    const double tauU = c.opk - c.omk * phC;
+    Un = UC + c.dt * (rhsU / tauU);
   }
-  const T phxn = (phR - phL) * (T)0.5;
-  const T phzn = (phT - phB) * (T)0.5;
-  const T psxn = (psR - psL) * (T)0.5;
-  const T pszn = (psT - psB) * (T)0.5;
-  T A2 = aniso_a(phxn, phzn, c);
+  const double phxn = (phR - phL) * 0.5;
+  const double phzn = (phT - phB) * 0.5;
+  const double psxn = (psR - psL) * 0.5;
+  const double pszn = (psT - psB) * 0.5;
+  double A2 = aniso_a(phxn, phzn, c);
   A2 = A2 * A2;
-  const T gradps2 = psxn * psxn + pszn * pszn;
-  const T extra = -c.sqrt2 * A2 * phC * gradps2;
-  const T Up = (T)(a.up_a + (double)gj * a.up_b);
-  const T rhs = ((JR - JL) + (JT - JB) + extra) * c.hi * c.hi + c.sqrt2 * phC -
-                c.lamd * ((T)1 - phC * phC) * c.sqrt2 * (Un + Up);
-  const T tp = (T)1 - c.omk * Up;
-  const T tau = ((tp >= c.k) ? tp : c.k) * A2;
-  const T dps = div_t(rhs, tau);
-  T noise = (T)0;
-  if (c.noise_amp != (T)0 && in_band(phC)) {
+  const double gradps2 = psxn * psxn + pszn * pszn;
+  const double extra = -c.sqrt2 * A2 * phC * gradps2;
+  const double Up = a.up_a + (double)gj * a.up_b;
+  const double rhs = ((JR - JL) + (JT - JB) + extra) * c.hi * c.hi + c.sqrt2 * phC -
+                     c.lamd * (1.0 - phC * phC) * c.sqrt2 * (Un + Up);
+  const double tp = 1.0 - c.omk * Up;
+  const double tau = ((tp >= c.k) ? tp : c.k) * A2;
+  const double dps = rhs / tau;
+  double noise = 0.0;
+  if (c.noise_amp != 0.0 && in_band(phC)) {
     const Philox4 rn = philox4x32_10((uint32_t)gi, (uint32_t)gj, a.step, 0x4E4F4953u, a.seed, 0x5EEDu);
-    noise = c.noise_amp * ((T)uniform01(rn.v[0]) - (T)0.5);
+    noise = c.noise_amp * (uniform01(rn.v[0]) - 0.5);
   }
-  const T psn = psC + c.dt * dps + noise;
-  V vps, vU, vD;
-  encode_cell<S>(a, merge, step_key, gi, gj, psn, Un, dps, vps, vU, vD);
-  put_with_halo(o_ps, o_U, o_D, a.pitch, a.fnx, a.fny, gj, gi, vps, vU, vD);
+  const double psn = psC + c.dt * dps + noise;
+  put_with_halo(o_ps, o_U, o_D, a.pitch, a.fnx, a.fny, gj, gi, psn, Un, dps);
 }
 
 // ---- register-marching step kernel ------------------------------------------
@@ -448,18 +440,15 @@ __device__ __forceinline__ MarchPos march_pos(int ngroups, int nchunks) {
 }
 
 // FP64 storage: one strip a warp, scalar arithmetic.
-template <class S>
 __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
-  using T = typename S::T;
-  using V = typename S::V;
-  const Consts<T> c = consts<T>(a);
+  const Consts c = consts(a);
   const bool merge = !a.prestep;
-  const V* in_ps = static_cast<const V*>(a.in);
-  const V* in_U = in_ps + a.plane;
-  const V* in_D = in_U + a.plane;
-  V* o_ps = static_cast<V*>(a.out);
-  V* o_U = o_ps + a.plane;
-  V* o_D = o_U + a.plane;
+  const double* in_ps = static_cast<const double*>(a.in);
+  const double* in_U = in_ps + a.plane;
+  const double* in_D = in_U + a.plane;
+  double* o_ps = static_cast<double*>(a.out);
+  double* o_U = o_ps + a.plane;
+  double* o_D = o_U + a.plane;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const MarchPos pos = march_pos((a.fnx - 2 + MW - 1) / MW, (a.fny - 2 + a.rows - 1) / a.rows);
@@ -469,11 +458,10 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
   const bool col_ok = gi < a.fnx;
   const bool out_col = lane >= 1 && lane <= MW && gi <= a.fnx - 2;
   const int y0 = 1 + pos.chunk * a.rows;
-  const uint32_t step_key = mix32(a.step ^ (a.seed * 0x9E3779B9u));
 
   // raw values of the next row to decode, loaded one row ahead of their use so
   // that the load latency overlaps the current row's arithmetic
-  V raw_ps{}, raw_U{}, raw_D{};
+  double raw_ps{}, raw_U{}, raw_D{};
   bool raw_ok = false;
   auto issue = [&](int r) {
     raw_ok = col_ok && r < a.fny;
@@ -484,21 +472,21 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
       raw_D = in_D[o];
     }
   };
-  auto load = [&](T& ps, T& ph, T& U, T& jat) {
-    ps = ph = U = jat = (T)0;
+  auto load = [&](double& ps, double& ph, double& U, double& jat) {
+    ps = ph = U = jat = 0.0;
     if (raw_ok) {
-      S::ld_pp(raw_ps, c.inv_sqrt2, ps, ph);
-      U = S::ldU(raw_U, c.U0);
-      jat = jat_of(c, U, ph, S::ld(raw_D));
+      StF64::ld_pp(raw_ps, c.inv_sqrt2, ps, ph);
+      U = StF64::ldU(raw_U, c.U0);
+      jat = jat_of(c, U, ph, StF64::ld(raw_D));
     }
   };
-  auto right = [&](T v) { return __shfl_down_sync(FULL, v, 1); };
-  auto left = [&](T v) { return __shfl_up_sync(FULL, v, 1); };
+  auto right = [&](double v) { return __shfl_down_sync(FULL, v, 1); };
+  auto left = [&](double v) { return __shfl_up_sync(FULL, v, 1); };
 
   // row r+1 ("c") and its right neighbour; row r ("b"); row r-1 ("a")
-  T ps_c, ph_c, U_c, j_c, Rps_c, Rph_c, RU_c, Rj_c;
-  T ps_b, ph_b, U_b, j_b, Rps_b, Rph_b, RU_b, Rj_b;
-  T ps_a, ph_a;
+  double ps_c, ph_c, U_c, j_c, Rps_c, Rph_c, RU_c, Rj_c;
+  double ps_b, ph_b, U_b, j_b, Rps_b, Rph_b, RU_b, Rj_b;
+  double ps_a, ph_a;
   auto fetch_c = [&]() {  // decode the issued row into "c"
     load(ps_c, ph_c, U_c, j_c);
     Rps_c = right(ps_c);
@@ -513,13 +501,13 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
     Rps_b = Rps_c; Rph_b = Rph_c; RU_b = RU_c; Rj_b = Rj_c;
   };
   // plaquette means at (x+1/2, r+1/2) from rows b and c
-  auto plaq = [&](T& qs, T& qp) {
-    qs = (((ps_b + Rps_b) + ps_c) + Rps_c) * (T)0.25;
-    qp = (((ph_b + Rph_b) + ph_c) + Rph_c) * (T)0.25;
+  auto plaq = [&](double& qs, double& qp) {
+    qs = (((ps_b + Rps_b) + ps_c) + Rps_c) * 0.25;
+    qp = (((ph_b + Rph_b) + ph_c) + Rph_c) * 0.25;
   };
   // y-edge (x, r+1/2) between rows b and c
-  auto yedge = [&](T qs, T qp, T& J, T& Uf) {
-    const T Lqs = left(qs), Lqp = left(qp);
+  auto yedge = [&](double qs, double qp, double& J, double& Uf) {
+    const double Lqs = left(qs), Lqp = left(qp);
     edge_flux<true>(c, merge, qs - Lqs, ps_c - ps_b, qp - Lqp, ph_c - ph_b, ph_b, ph_c, U_b, U_c,
                     j_b, j_c, J, Uf);
   };
@@ -533,9 +521,9 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
   issue(y0);
   fetch_c();
   issue(y0 + 1);
-  T qs_hi, qp_hi;
+  double qs_hi, qp_hi;
   plaq(qs_hi, qp_hi);
-  T yJ_hi, yU_hi = (T)0;
+  double yJ_hi, yU_hi = 0.0;
   yedge(qs_hi, qp_hi, yJ_hi, yU_hi);
 
   for (int t = 0; t < a.rows; ++t) {
@@ -544,20 +532,19 @@ __global__ void __launch_bounds__(MWARPS * 32) ek2d_march_kernel(EkArgs a) {
     shift();
     fetch_c();      // row r+1, issued one row earlier
     issue(r + 2);   // in flight during this row's arithmetic
-    const T qs_lo = qs_hi, qp_lo = qp_hi;
+    const double qs_lo = qs_hi, qp_lo = qp_hi;
     plaq(qs_hi, qp_hi);
     // x-edge (x+1/2, r)
-    T xJ, xU = (T)0;
+    double xJ, xU = 0.0;
     edge_flux<false>(c, merge, Rps_b - ps_b, qs_hi - qs_lo, Rph_b - ph_b, qp_hi - qp_lo, ph_b, Rph_b,
                      U_b, RU_b, j_b, Rj_b, xJ, xU);
-    const T yJ_lo = yJ_hi, yU_lo = yU_hi;
+    const double yJ_lo = yJ_hi, yU_lo = yU_hi;
     yedge(qs_hi, qp_hi, yJ_hi, yU_hi);
-    const T xJ_L = left(xJ), xU_L = left(xU);
-    const T Lps = left(ps_b), Lph = left(ph_b);
+    const double xJ_L = left(xJ), xU_L = left(xU);
+    const double Lps = left(ps_b), Lph = left(ph_b);
     if (out_col)
-      cell_update<S>(a, c, merge, step_key, gi, r, ps_b, ph_b, U_b, j_b, xJ, xJ_L, yJ_hi, yJ_lo, xU,
-                     xU_L, yU_hi, yU_lo, Rph_b, Lph, ph_c, ph_a, Rps_b, Lps, ps_c, ps_a, o_ps, o_U,
-                     o_D);
+      cell_update(a, c, merge, gi, r, ps_b, ph_b, U_b, j_b, xJ, xJ_L, yJ_hi, yJ_lo, xU, xU_L, yU_hi,
+                  yU_lo, Rph_b, Lph, ph_c, ph_a, Rps_b, Lps, ps_c, ps_a, o_ps, o_U, o_D);
   }
 }
 
