@@ -31,12 +31,12 @@ struct NuclArgs {
   const float* sphere;  // (2*pts+1)^3 nucleus profile: tanh(dx*((1+pts)/2 - r)/sqrt2)
   int* status;          // per coarse cell: 1 = solid / already nucleated
   int* count;           // nucleation events (accumulated)
-  // quiet-item flags of the buffer written (NULL = none kept): the items a
-  // nucleus reaches are marked not quiet; tile tw x th cells, z chunk zc
   // change marks of the buffer written (NULL = none kept): a nucleus changes the
-  // id lists of its cells (mark_readers, apt_step.cuh)
+  // id lists of its cells (mark_readers, apt_common.cuh)
   uint8_t* redo;
   int bcX, bcY, bcZ;
+  // quiet-item flags of the buffer written (NULL = none kept): the items a
+  // nucleus reaches are marked not quiet; tile tw x th cells, z chunk zc
   uint8_t* quiet;
   int tw, th, zc, ntx, nty;
 };

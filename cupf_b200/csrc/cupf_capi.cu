@@ -439,24 +439,6 @@ static int resident_per_sm(const cupf_apt_handle* h, int ty) {
   return r;
 }
 
-// Default z-chunk of a work item: the largest of 16, 8, 4, 2, 1 planes that
-// still gives at least 2.5 work items per resident CTA, else 1.  Measured on
-// the line case (B200, NUM_PF = 5 and 8): 16 is best from 128x128x256 up, while
-// 96^3 wants 4 and 64^3 or 48^3 want 1-2 (2.5-3x faster than 8 there) -- with
-// fewer items than CTAs most of the GPU idles, with many short items each pays
-// the two extra planes of its TMA pipeline fill.
-static int default_zc(cupf_apt_handle* h) {
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-  const long long tiles =
-      (long long)((h->p.fnx - 2 + TX - 1) / TX) * ((h->p.fny - 2 + h->ty - 1) / h->ty);
-  const int nz = h->p.fnz - 2;
-  const long long want = (5LL * resident_per_sm(h, h->ty) * nsm + 1) / 2;
-  for (int zc = 16; zc > 1; zc /= 2)
-    if (tiles * ((nz + zc - 1) / zc) >= want) return zc;
-  return 1;
-}
-
 // Work-item shape for a state whose grain ids occupy nz_active interior planes (those
 // within 10 planes of a plane holding an id: the tails the first steps grow).  Quiet
 // items cost next to nothing, so the items that count are the ones the step computes.
@@ -631,7 +613,7 @@ extern "C" cupf_status cupf_apt_create(const cupf_apt_params* p, const cupf_apt_
   TRY(alloc_maps(h));  // last: takes only room the rest left
   const char* zc_env = getenv("CUPF_ZC");
   h->zc_user = zc_env != nullptr;
-  set_zc(h, zc_env ? atoi(zc_env) : default_zc(h));
+  set_zc(h, zc_env ? atoi(zc_env) : 16);  // chosen when a state is loaded (choose_shape)
   TRY(cuda(cudaStreamSynchronize(h->stream), "sync"));
 #undef TRY
   *out = h;
