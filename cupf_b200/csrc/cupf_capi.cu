@@ -817,6 +817,11 @@ extern "C" cupf_status cupf_apt_step(cupf_apt_handle* h, int32_t nsteps,
   if (nsteps < 0) return fail(CUPF_ERR_INVALID, "nsteps < 0");
   std::lock_guard<std::recursive_timed_mutex> use(h->map_use);
   CK(cudaSetDevice(h->device));
+  // a caller that captures the steps in a graph keeps the maps' addresses in it: they are
+  // no longer given back to other allocations
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (h->map) CK(cudaStreamIsCapturing(h->stream, &capture));
+  if (capture == cudaStreamCaptureStatusActive) forget_map_owner(h);
   for (int n = 0; n < nsteps; ++n) {
     // t of step m (1-based): (float)m * dt * tau0, as (2*kt+1)*dt*tau0 in evolve
     const float t = (float)(h->steps_done + 1) * h->p.dt * h->p.tau0;

@@ -242,6 +242,34 @@ def maps_give_way_across_threads():
         equal(s.collect(clear=True), want)
 
 
+def captured_steps_keep_their_maps():
+    """Steps captured in a graph on the handle's stream: the maps they point to are not
+    given back afterwards, and the graph's steps are the steps."""
+    a, c = shim(), line()
+    with APTSolver(c) as s:
+        s.init_from_argmax(c.phi, c.alpha)
+        s.step(12)
+        want = s.get_slots()
+    rt = C.CDLL("libcudart.so.12")
+    graph, run = C.c_void_p(), C.c_void_p()
+    with APTSolver(c) as s:
+        s.init_from_argmax(c.phi, c.alpha)
+        s.step(10)
+        s.sync()
+        stream = C.c_void_p(s.stream)
+        assert rt.cudaStreamBeginCapture(stream, 2) == 0  # relaxed
+        s.step(2)
+        assert rt.cudaStreamEndCapture(stream, C.byref(graph)) == 0
+        assert rt.cudaGraphInstantiate(C.byref(run), graph, C.c_ulonglong(0)) == 0
+        live = a.alloc_live()
+        refused(a, 0, s.get_slots)
+        assert a.alloc_live() == live
+        assert rt.cudaGraphLaunch(run, stream) == 0
+        s.sync()
+        same(s.get_slots(), want)
+        assert rt.cudaGraphExecDestroy(run) == 0 and rt.cudaGraphDestroy(graph) == 0
+
+
 def forms_of_the_merge():
     """Crowded lists (holes, repeated ids, more grains than slots) with and without maps:
     rows merged by the warp's passes, by their own lanes, and both."""
@@ -269,7 +297,7 @@ def forms_of_the_merge():
 
 
 @pytest.mark.parametrize("name", ["maps_give_way", "maps_give_way_across_threads",
-                                  "forms_of_the_merge"])
+                                  "captured_steps_keep_their_maps", "forms_of_the_merge"])
 def test_slot_maps_give_way(child, name):
     child(name)
 
