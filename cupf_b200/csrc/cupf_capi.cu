@@ -448,8 +448,11 @@ static int resident_per_sm(const cupf_apt_handle* h, int ty) {
 //     NUM_PF = 5 and 8), for its finer items: 117x75x139 NUM_PF = 6 59 against 65.
 //     16-bit pairs keep 8, whose centre plane is decoded once: 128x128x256 149 against
 //     154, 192^3 240 against 245;
-//   any format takes 4 where the 32x8 tiles would need chunks of one plane to give every
-//     CTA two items: 24x24x32 FP32 14.2 against 16.0;
+//   any format takes 4 where its items in chunks of one plane exceed its resident CTAs by
+//     no more than a fifth (some of the counted planes hold nothing yet), so that the finer
+//     items cost no second turn: NUM_PF = 8 FP32 32x64x64 16.0 against 17.0, 40^3 14.9
+//     against 15.9, but 48^3, past the line, 18.5 against 16.5 and 64x64x128 42.7 against
+//     35.5; NUM_PF = 5 24x24x32 13.6 against 15.0, 100x30x60 17.2 against 18.5;
 //   z chunk: the largest of 16, 8, 4, 2 that gives 2 (tile height 8) or 1.75 (4) items
 //     per resident CTA over the active planes, else 1.
 static cupf_status choose_shape(cupf_apt_handle* h, int nz_active) {
@@ -460,7 +463,7 @@ static cupf_status choose_shape(cupf_apt_handle* h, int nz_active) {
   };
   const int r8 = resident_per_sm(h, 8), r4 = resident_per_sm(h, 4);
   if (!h->ty_user) {
-    const bool few = tiles(8) * ((nz_active + 1) / 2) < 2LL * r8 * nsm;
+    const bool few = tiles(4) * nz_active <= 6LL * r4 * nsm / 5;
     const int ty = few || (h->pair_bytes == 8 && 4 * r4 >= 8 * r8) ? 4 : 8;
     if (ty != h->ty) {
       h->ty = ty;
