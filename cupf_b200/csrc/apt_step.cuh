@@ -33,8 +33,8 @@
 // marks the cells that read it (mark_readers) for the next step; whoever replaces
 // the whole state invalidates every map.  A few marked cells are merged by the warp
 // together, four a pass with a lane per stencil point, so that scattered cells do not
-// hold up a warp's other lanes; a row that is nearly all marked by its own lanes
-// (kRowMerge), as every row is where the device has no room for maps.
+// hold up a warp's other lanes; a row with many by its own lanes (row_merge), as every
+// row is where the device has no room for maps.
 //
 // What bounds it: instruction issue and latency, not bytes.  128x128x256 line case, NUM_PF
 // = 8, on a B200, us per step over steps 1-20, 21-50 and 51-150 (all-empty items left
@@ -317,11 +317,39 @@ __device__ __forceinline__ uint2 merge_cell(const typename S::T* pD, const typen
   return make_uint2(info | ((uint32_t)cnt << 28), al);
 }
 
-// The same out of line, where it runs seldom.
+// The same out of line.
 template <int NP, class S, int BW, int BCELLS>
 __device__ __noinline__ uint2 merge_cell_call(const typename S::T* pD, const typename S::T* pC,
                                               const typename S::T* pU, uint32_t* wcol) {
   return merge_cell<NP, S, BW, BCELLS>(pD, pC, pU, wcol);
+}
+
+// A row with more marked cells than this is merged by its own lanes; 0: by the warp's
+// passes whatever their number, as long as maps are kept.  The line lies where a row by
+// its own lanes costs what its passes do: the fewer the slots, the cheaper the former, and
+// with up to three the passes are not built at all (most cells of an interface then
+// overflow and are merged every step).  Measured on a B200, us per step over the first 20
+// steps and over steps 51-150:
+//   NUM_PF = 8 FP32, passes only -> 28: line 128x128x256 233, 164 -> 220, 163; pool
+//     256x256x768 5380, 4673 -> 5200, 4620.  16-bit pairs there keep to the passes, since
+//     the pool's FP64 model leaves little of the instruction cache: 28 marks 5241, 4597
+//     against 5114, 4414 (line 198, 144 against 202, 144);
+//   28 -> this, FP32: NUM_PF = 6 200x150x100 150.4, 112.7 -> 149.9, 112.6; 5 128^3 90.8, 73.5
+//     -> 89.3, 73.4; 4 160x128x128 96.3, 82.0 -> 94.3, 81.1; 3 128^3 74.3, 67.1 -> 67.3, 61.8;
+//     2 62.7, 56.9 -> 54.4, 50.2; 1 47.6, 45.1 -> 45.3, 42.8;
+//   never -> this, FP16: 7 160x160x128 164.5, 120.8 -> 158.9, 121.1; 6 141.5, 100.5 -> 133.8,
+//     100.7; 5 98.4, 76.0 -> 92.9, 76.0; 4 109.0, 87.8 -> 99.2, 87.3; 3 84.7, 72.7 -> 72.0,
+//     66.2; 2 72.4, 62.1 -> 58.7, 54.6; 1 56.3, 48.9 -> 46.3, 43.8.
+// Without maps (NUM_PF = 8, steps 51-150): FP32 line 317 with passes, 286 by lanes, pool
+// 7611 and 5894; FP16 276 and 242, 7000 and 5667.
+template <int NP, class S>
+constexpr int row_merge() {
+  return NP <= 3 ? 0
+         : NP == 4 ? 12
+         : NP == 5 ? 20
+         : NP == 6 ? (S::kBytes == 8 ? 24 : 20)
+         : NP == 7 ? (S::kBytes == 8 ? 28 : 24)
+                   : (S::kBytes == 8 ? 28 : 0);
 }
 
 // One work item: the column tile (txi, tyi) over the z chunk zci of one
@@ -339,16 +367,7 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
   constexpr int BW = Smem::BW;
   constexpr int BCELLS = Smem::BCELLS;
   constexpr bool kDec = Smem::kDecode;
-  // A row with more marked cells than this is merged by its own lanes, at about the cost
-  // of seven passes of four cells (0: only where no maps are kept).  Measured on a B200, us
-  // per step over the first 20 steps and over steps 51-150, NUM_PF = 8: FP32 28: line
-  // 128x128x256 220 and 163, pool 256x256x768 5200 and 4620; 24: 222, 163, 5216, 4632; with
-  // passes only 233, 164, 5380, 4673.  In 16-bit pairs, whose pool's FP64 model leaves little
-  // of the instruction cache, 28: 198, 144, 5241, 4597, with passes only 202, 144, 5114, 4414;
-  // there it is a call, too: inline it costs the pool 4963 where it is never taken.
-  // Without maps: FP32 line 317 with passes only, 286 by lanes, pool 7611 and 5894; FP16
-  // 276 and 242, 7000 and 5667.
-  constexpr int kRowMerge = S::kBytes == 8 ? 28 : 0;
+  constexpr int kRowMerge = row_merge<NP, S>();
   constexpr unsigned FULL = 0xffffffffu;
   // offsets of the centre plane's stencil points B, L, C, R, T from the cell
   constexpr int ctr_off[7] = {0, -BW, -1, 0, 1, BW, 0};
@@ -512,10 +531,12 @@ __device__ __forceinline__ void step_item(const CUtensorMap* tmap, const StepArg
     bool force_mark = false;
     uint32_t todo = __ballot_sync(FULL, need);
     uint32_t info = 0;
-    if (todo && (!a.map || (kRowMerge && __popc(todo) > kRowMerge))) {
+    if (todo && (NP <= 3 || !a.map || (kRowMerge && __popc(todo) > kRowMerge))) {
       if (need) {  // most of the row, or every cell of every step: a lane per cell
         uint2 r;
-        if constexpr (kRowMerge != 0)
+        // inline where that is the faster (NUM_PF = 5 FP32, 64^3: 16.6 against 16.9; the
+        // other way round 4 FP32, 96^3: 39.8 against 38.4, and the pool in 16-bit pairs)
+        if constexpr ((S::kBytes == 8 && NP >= 5) || NP <= 3)
           r = merge_cell<NP, S, BW, BCELLS>(plD + c, stC + c, plU + c, wcol);
         else
           r = merge_cell_call<NP, S, BW, BCELLS>(plD + c, stC + c, plU + c, wcol);
