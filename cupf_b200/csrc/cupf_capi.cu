@@ -379,7 +379,11 @@ bool release_slot_maps() {
     cupf_apt_handle* h = g_map_owners[i];
     if (h->device != device) continue;
     std::unique_lock<std::recursive_timed_mutex> use(h->map_use, std::chrono::seconds(1));
-    if (!use || cudaStreamSynchronize(h->stream) != cudaSuccess) continue;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+    if (!use || cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess ||
+        capture != cudaStreamCaptureStatusNone)
+      continue;  // in a call of another thread, or being captured (a wait would break that)
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess) continue;
     free_maps(h);
     g_map_owners.erase(g_map_owners.begin() + i);
     return true;

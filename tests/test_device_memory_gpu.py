@@ -258,7 +258,9 @@ def captured_steps_keep_their_maps():
         s.sync()
         stream = C.c_void_p(s.stream)
         assert rt.cudaStreamBeginCapture(stream, 2) == 0  # relaxed
-        s.step(2)
+        with APTSolver(c) as other:  # created while the stream is being captured
+            refused(a, 0, other.set_slots, *want)
+            s.step(2)
         assert rt.cudaStreamEndCapture(stream, C.byref(graph)) == 0
         assert rt.cudaGraphInstantiate(C.byref(run), graph, C.c_ulonglong(0)) == 0
         live = a.alloc_live()
